@@ -123,7 +123,9 @@ def _reflectors(n, g):
     sweep = torch.arange(n, device=DEV)[:, None]
     length = -(-n // b) * b
     P = torch.randn(n, length, generator=g, dtype=F64, device=DEV)  # row s: sweep s from row s + 1
-    P *= (torch.arange(length, device=DEV)[None, :] < n - sweep - 1) & (sweep < n - 2)
+    # (a segment of one row would start at row n - 1: the chase stores none there)
+    last = torch.where((n - 2 - sweep) % b == 0, n - sweep - 2, n - sweep - 1)
+    P *= (torch.arange(length, device=DEV)[None, :] < last) & (sweep < n - 2)
     P = P.view(n, length // b, b)
     P *= torch.sqrt(2.0 / (P * P).sum(dim=2, keepdim=True).clamp_min(1e-300))
     at = torch.arange(n, device=DEV)[None, :] - sweep - 1
