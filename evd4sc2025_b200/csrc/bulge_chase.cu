@@ -1,4 +1,5 @@
-// Stage 2: band -> tridiagonal bulge chasing, persistent sm_100a kernel.
+// Stage 2: band -> tridiagonal bulge chasing: the entry points, and the
+// kernel for orders beyond the reach of the pipeline kernel (chase_pipe.cu).
 //
 // Algorithm (same reflectors, same storage as chasing_kernel_one_timeV10,
 // util/inc/bugle_chasingV10.h:21-392): sweep s (s = 0..n-3) annihilates column
@@ -33,6 +34,10 @@
 #include "common.cuh"
 
 namespace evd {
+
+long chase_pipe_ints(long n);
+int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* msg, long s0,
+                      long s1, cudaStream_t st, bool* used);
 
 namespace {
 
@@ -345,7 +350,8 @@ int band_pack(long n, long b, const double* dA, long ldA, double* dSub, long ldS
   return EVD_SUCCESS;
 }
 
-long chase_iwork_ints(long n) { return n + 64; }
+// flags, tickets and the error word, then the pipeline's boundary messages
+long chase_iwork_ints(long n) { return n + 64 + chase_pipe_ints(n); }
 
 // Sweeps [s0, s1) of the chase as one launch (part `part`, 0 <= part < 32, of
 // a chase split into consecutive ranges; part 0 starts at s0 = 0 and clears
@@ -369,6 +375,9 @@ int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long 
   if (part == 0) EVD_CUDA_TRY(cudaMemsetAsync(iwork, 0, sizeof(int) * chase_iwork_ints(n), st));
   s1 = std::min(s1, n - 2);
   if (s1 > s0) {
+    bool used = false;
+    EVD_TRY(launch_chase_pipe(n, dSub, dU, ldU, err, iwork + n + 64, s0, s1, st, &used));
+    if (used) return EVD_SUCCESS;
     // enough CTAs for the pipeline's concurrency (a sweep starts every 3 steps
     // and lasts about n/b steps), bounded by the GPU's resident capacity
     const long sweeps = s1 - s0;
@@ -444,14 +453,15 @@ extern "C" int evd_bulge_chase(long n, long b, double* dSub, long ldSub, double*
 // plugin running inside a host framework that owns the allocator), and
 // loops that are required to run with a fixed memory footprint.  For them the
 // scratch lives in a file-scope device array instead, sized for bands of up
-// to kNoAllocMaxN columns (256 KB that every GPU loading this library keeps
+// to kNoAllocMaxN columns (600 KB that every GPU loading this library keeps
 // until the process exits).
 namespace evd {
 
 constexpr long kNoAllocMaxN = 65536;
+constexpr long kNoAllocMsgInts = 84000;  // >= chase_pipe_ints of every order
 constexpr int kNoAllocMaxDevices = 64;
 
-static __device__ __align__(256) int g_chase_noalloc_scratch[kNoAllocMaxN + 64];
+static __device__ __align__(256) int g_chase_noalloc_scratch[kNoAllocMaxN + 64 + kNoAllocMsgInts];
 
 // Device address of the scratch on the current device.  In host code the
 // array's name is only a host-side stand-in, so the address is looked up with
@@ -488,6 +498,7 @@ extern "C" int evd_bulge_chase_noalloc(long n, long b, double* dSub, long ldSub,
             evd::kNoAllocMaxN, n);
     return EVD_ERR_INVALID_ARG;
   }
+  if (n > 0 && evd::chase_pipe_ints(n) > evd::kNoAllocMsgInts) return EVD_ERR_INVALID_ARG;
   int* iw = nullptr;
   EVD_TRY(evd::chase_noalloc_scratch(&iw));
   // bulge_chase_async clears the flags, ticket and error word of the scratch

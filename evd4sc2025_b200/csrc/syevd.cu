@@ -46,6 +46,7 @@ int q2_apply(bool forward, long n, long ncols, const double* U, long ldU, double
              double* tbuf, cudaStream_t st);
 int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, double* X,
                    long ldX, double* tbuf, long h0, long h1, long ident_k, cudaStream_t st);
+bool chase_pipelined(long n);
 int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, int* iwork,
                      long s0, long s1, int part, cudaStream_t st);
 int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, cudaStream_t st);
@@ -284,11 +285,11 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
 
 size_t syevd_ws_bytes(long n, long b, long nb) { return layout(n, b, nb).bytes; }
 
-// Sweep ranges of the pipelined chase.  Below the split sweep k (a multiple
-// of 8): [0, 512), [512, 1536), ... doubling, the last one ending at k; from k
-// on: ranges of max(2048, (n - 2 - k) / 16) sweeps (rounded up to a multiple
-// of 8), the last one ending at sweep n - 2.  k = 0: no lower part.  Returns
-// the number of ranges r (at most 32); range i is [bounds[i], bounds[i+1]).
+// Sweep ranges of a chase too long for the pipeline kernel (n > 33000 or so):
+// [0, 512), [512, 1536), ... doubling up to k, then max(2048, (n - 2 - k) / 16)
+// sweeps each, the last one ending at sweep n - 2, so that stage 2 can follow
+// one range behind.  k = 0: no lower part.  Returns the number of ranges r (at
+// most 32); range i is [bounds[i], bounds[i+1]).
 static int chase_ranges(long n, long k, long bounds[34]) {
   const long S = std::max(n - 2, 0L);
   int c = 0;
@@ -310,21 +311,30 @@ static int chase_ranges(long n, long k, long bounds[34]) {
   return c;
 }
 
-// The mixed form with the stage-2 reflectors applied while the chase runs.
-// Q2^T = B A with A = the reflectors of the sweeps [0, k) and B those of the
-// sweeps [k, n - 2), each accumulated from the identity by the DMMA stage-2
-// kernel one chase range behind the chase (a CTA skips the strips that are
-// still zero below its columns).  The kernel's dependency chain (strips x
-// blocks of 8 sweeps per column) is the longest path of the solve; splitting
-// it at k = 0.39 n into two chains that run side by side about halves it
-// (A starts after the first range, B once the chase has passed k).
-//   main:   sy2sb (emulated trailing SYR2K) -> band pack -> chase, one launch
-//           per sweep range -> D&C (own integer workspace; Z into W once the
-//           Q1 formation no longer reads W)
+// The whole chase as one range.
+static int one_range(long n, long bounds[34]) {
+  bounds[0] = 0;
+  bounds[1] = std::max(n - 2, 0L);
+  return 1;
+}
+
+// The mixed form.  Q2^T = B A with A = the reflectors of the sweeps [0, k) and
+// B those of the sweeps [k, n - 2), each accumulated from the identity by the
+// DMMA stage-2 kernel (a CTA skips the strips that are still zero below its
+// columns) after the chase, beside the divide and conquer and the Q1 formation.
+// That kernel's dependency chain (strips x blocks of 8 sweeps per column) is
+// the longest path of the solve; two chains that run side by side halve it.
+// For the heaviest column their lengths are k (n - k) + k^2 / 2 and
+// (n - k)^2 / 2 in units of sweep-strips, equal at k = (1 - sqrt(1/2)) n.
+// The chains used to follow the chase one sweep range behind; since the chase
+// takes 41 ms of the solve at n = 16384 (181 ms before the pipeline kernel)
+// running it first, alone and in one launch, is faster (876 against 948 ms).
+//   main:   sy2sb (emulated trailing SYR2K) -> band pack -> chase -> D&C (own
+//           integer workspace; Z into W once the Q1 formation no longer reads W)
 //   side B: slab merge, Q1 formed explicitly (emulated)
-//   side A: A = I, the ranges below k; T1 = A Q1^T; Q^T = B T1;
+//   side A: A = I, the sweeps below k; T1 = A Q1^T; Q^T = B T1;
 //           X = Q Z (emulated, the main integer workspace)
-//   side C: B = I, the ranges from k
+//   side C: B = I, the sweeps from k
 // Without the extra n x n buffer (orders above kMixedDcOwnMax) there is one
 // chain, P = Q2^T in X, then Y2 = P^T Z and X = Q1 Y2.
 // Buffers: A in the extra buffer (then Q^T), B (or P) in X, Q1 in dA, T1 (or
@@ -355,7 +365,7 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
   double* tbuf = ((size_t)q2_tbuf_doubles(n) <= (size_t)n * n) ? OA : nullptr;
   double* XA = mx->split_buf;  // chain A, then Q^T
   const bool split = XA != nullptr && n > 64;
-  const long k = split ? std::max(8L, (long)(0.39 * (double)n) / 8 * 8) : 0;
+  const long k = split ? std::max(8L, (long)(0.293 * (double)n) / 8 * 8) : 0;
   SideStream sideA, sideB, sideC;
   EVD_TRY(sideA.init(timed != 0));
   EVD_TRY(sideB.init(timed != 0));
@@ -368,7 +378,7 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
   cudaEvent_t* ev = sideA.ev;
   cudaEvent_t* evr = sideB.ev;
   long bounds[34];
-  const int nr = chase_ranges(n, k, bounds);
+  const int nr = chase_pipelined(n) ? one_range(n, bounds) : chase_ranges(n, k, bounds);
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[0], st));
   {
     NvtxRange r("evd_b200 sy2sb (emulated trailing update)");
@@ -420,11 +430,13 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
   {
     NvtxRange r("evd_b200 stage-2 reflectors beside the chase (side streams)");
     for (int i = 0; i < nr; ++i) {
-      const bool in_b = split && bounds[i] >= k;
-      cudaStream_t s2 = in_b ? sc : sa;
-      EVD_CUDA_TRY(cudaStreamWaitEvent(s2, evr[i], 0));
-      EVD_TRY(q2_apply_range(true, n, n, U, n, in_b ? X : PA, in_b ? ldX : ldPA, tbuf,
-                             bounds[i], bounds[i + 1], in_b ? k : 0, s2));
+      EVD_CUDA_TRY(cudaStreamWaitEvent(sa, evr[i], 0));
+      EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, bounds[i],
+                             split ? k : bounds[i + 1], 0, sa));
+      if (split) {
+        EVD_CUDA_TRY(cudaStreamWaitEvent(sc, evr[i], 0));
+        EVD_TRY(q2_apply_range(true, n, n, U, n, X, ldX, tbuf, k, bounds[i + 1], k, sc));
+      }
     }
   }
   EVD_CUDA_TRY(cudaEventRecord(ev[5], sa));

@@ -147,7 +147,7 @@ int evd_bulge_chase(long n, long b, double* dSub, long ldSub, double* dU, long l
  * cudaMalloc allowed there: a fixed memory footprint, or a host framework that
  * owns the allocator).  This entry point has no counterpart in the reference.
  * Its scratch is a file-scope device array of the library, sized for
- * n <= 65536 (256 KB per GPU that loads the library, kept until exit); larger
+ * n <= 65536 (600 KB per GPU that loads the library, kept until exit); larger
  * n is rejected with EVD_ERR_INVALID_ARG and a message on stderr.  The first
  * call on a device looks up the array's device address (cudaGetSymbolAddress);
  * make that first call before any stream capture.  Every call shares the one
@@ -304,10 +304,9 @@ int evd_syevd_batched(long count, const long* n, const double* const* A, const l
  * Then `refine_iters` Ogita-Aishima iterations with FP64-level emulated
  * products win FP64 accuracy back (the X E update uses `moduli_update`,
  * <= 14).
- * The chase runs as consecutive sweep ranges.  The DMMA stage-2 kernel
- * accumulates A (the reflectors of the sweeps below 0.39 n) and B (the rest)
- * from the identity on side streams, one range behind the chase.  The Q1
- * formation and the divide and conquer run beside them.  Up to n = 24576
+ * After the chase the DMMA stage-2 kernel accumulates A (the reflectors of
+ * the sweeps below 0.293 n) and B (the rest) from the identity on side
+ * streams.  The Q1 formation and the divide and conquer run beside them.  Up to n = 24576
  * the work size includes an n x n buffer and integer workspaces of their own
  * for the divide and conquer and the Q1 formation.  The panels, the chase,
  * the divide and conquer and the stage-2 reflectors are the plain FP64

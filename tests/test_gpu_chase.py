@@ -73,3 +73,29 @@ def test_chase_repeatable(cuda, evdlib):
         out.append((d.clone(), e.clone(), U.clone()))
     torch.cuda.synchronize()
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("n", [130, 131, 259, 515, 1027, 2050, 2051, 18950])
+def test_chase_is_an_orthogonal_similarity(cuda, evdlib, n):
+    """B Q2 Z = Q2 T Z on a few random vectors, at the orders where the chase
+    changes its form (one CTA, clusters of 2 to 16, cooperative launches)."""
+    b = 32
+    g = torch.Generator(device=cuda).manual_seed(n)
+    sub = torch.zeros(n, 2 * b, dtype=torch.float64, device=cuda)
+    for o in range(b + 1):
+        sub[: n - o, o] = torch.randn(n - o, generator=g, dtype=torch.float64, device=cuda)
+    band = sub.clone()
+    d, e, U = evdlib.bulge_chase(sub.t(), b)
+    Z = evdlib.to_cm(torch.randn(n, 4, generator=g, dtype=torch.float64, device=cuda), device=cuda)
+    TZ = d[:, None] * Z
+    TZ[1:] += e[:, None] * Z[:-1]
+    TZ[:-1] += e[:, None] * Z[1:]
+    QTZ = evdlib.bc_back_apply(evdlib.to_cm(TZ, device=cuda), U)
+    QZ = evdlib.bc_back_apply(Z.clone(memory_format=torch.preserve_format), U)
+    BQZ = band[:, :1] * QZ
+    for o in range(1, b + 1):
+        BQZ[o:] += band[: n - o, o: o + 1] * QZ[: n - o]
+        BQZ[: n - o] += band[: n - o, o: o + 1] * QZ[o:]
+    # backward stable: a few units of rounding per reflector that a row meets
+    norm2 = 2.0 * 65 ** 0.5  # of a random band matrix, from above to within a factor of 2
+    assert (BQZ - QTZ).norm() <= 8e-13 * norm2 * Z.norm()
