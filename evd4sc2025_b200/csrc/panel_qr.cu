@@ -15,13 +15,17 @@
 //    and the last child to arrive at a parent (atomic counter) goes on to
 //    factor the parent.  Nobody waits, so there is no grid barrier and no
 //    spin.  The reference launches one kernel plus batched GEMMs per level.
-//  * One finishing kernel forms each tile's rows of the explicit thin Q
-//    (leaf Q times the 32x32 path product down the tree, right to left as
-//    the reference's recursion), and in the same pass rebuilds the Householder
-//    form: the unpivoted LU of (I - Q)[0:32] (recomputed redundantly by each
-//    CTA from tile 0's data, so no inter-CTA dependency), Y = (I-Q) U^{-1}
-//    (rows >= 32) or L1 (rows < 32), W = (I-Q) L1^{-T}.  This replaces the
-//    getrf + getLower + trsm + copy kernels.
+//  * tsqr_q_kernel forms the explicit thin Q of all nodes at once from their
+//    reflectors V (128 x 32, every tau = 1): Q_node = E - V K, E = [I; 0],
+//    K = T V_top^T, T^-1 = I + striu(V^T V): a Gram matrix on DMMA, one
+//    triangular solve, one DMMA product.
+//  * The finishing kernel multiplies 32 x 32 blocks down the tree (right to left
+//    as the reference's recursion): a leaf's rows of the thin Q are Q_leaf M.
+//    Every CTA also walks to leaf 0 and factors (I - Q)[0:32] = L1 U there
+//    (redundantly, no inter-CTA dependency), inverts both factors, and forms
+//    Y = (I - Q) U^{-1} and W = (I - Q) L1^{-T} of its 128 rows as one
+//    128 x 32 x 64 DMMA product.  This replaces the reference's getrf +
+//    getLower + trsm + copy kernels.  Figures: at panel_qr_launch.
 //  * In the sy2sb pipeline the finishing kernel writes Y and W straight into
 //    dY/dW and the band (R over zeros) into dA (the reference's copyMatrix +
 //    getU, api/zy_zy_sy2sb.cu:122-125).
@@ -35,9 +39,7 @@ namespace {
 constexpr int kTile = 128;        // rows per TSQR tile (reference: M = 128)
 constexpr int kNB = 32;           // panel width (reference: N = 32)
 constexpr int kFan = kTile / kNB; // children per tree node (their R factors fill one tile)
-constexpr int kThreads = 256;     // 8 warps x 4 columns
-constexpr int kRPL = kTile / 32;  // rows per lane in a tile QR
-constexpr int kSub = 128;         // rows per CTA of the finishing kernel
+constexpr int kThreads = 256;     // up-sweep: 8 warps x 4 columns
 constexpr int kMaxLevels = 16;
 
 struct TsqrPlan {
@@ -47,7 +49,7 @@ struct TsqrPlan {
   int rows[kMaxLevels];     // rows of the matrix factored at each level
   long soff[kMaxLevels];    // offset (doubles) of stack S_L in ws (L >= 1)
   int coff[kMaxLevels];     // offset of the arrival counters of level L (L >= 1)
-  long qtop_off;            // 32x32 copy of tile 0's leaf Q rows 0..31
+  long qtop_off;            // 32x32 copy of the top of leaf 0's Q, row-major
   long cnt_off;             // int counters start (in doubles, aligned)
   int ncnt;
   long total;               // doubles
@@ -86,235 +88,134 @@ TsqrPlan make_plan(long m) {
   return p;
 }
 
-// Full warp sums of four per-lane partials (one per column of the warp):
-// reduce-scatter (lanes keep two columns, then one) and a broadcast back, 20
-// 32-bit shuffles instead of 40 for four butterflies.
-__device__ __forceinline__ void warp_sum4(double (&p)[4], int lane) {
-  const bool b4 = lane & 16, b3 = lane & 8;
-  const double s0 = b4 ? p[0] : p[2], s1 = b4 ? p[1] : p[3];
-  const double r0 = __shfl_xor_sync(0xffffffffu, s0, 16);
-  const double r1 = __shfl_xor_sync(0xffffffffu, s1, 16);
-  const double k0 = (b4 ? p[2] : p[0]) + r0;  // column 2*b4
-  const double k1 = (b4 ? p[3] : p[1]) + r1;  // column 2*b4 + 1
-  const double r = __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
-  double k = (b3 ? k1 : k0) + r;  // column 2*b4 + b3
-  k += __shfl_xor_sync(0xffffffffu, k, 4);
-  k += __shfl_xor_sync(0xffffffffu, k, 2);
-  k += __shfl_xor_sync(0xffffffffu, k, 1);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) p[c] = __shfl_sync(0xffffffffu, k, (c >> 1) * 16 + (c & 1) * 8);
-}
-
 // Householder QR of one tile (mm <= 128 rows, 32 columns) held in registers:
-// warp w owns columns w, w + 8, w + 16, w + 24 (a[c] holds column 8c + w),
-// lane l owns rows l + 32 i (i < 4).  Writes R (32 x 32, upper; diag =
-// -sign(x0) ||x||) to Rdst and leaves the reflectors in the tile (column j,
-// rows >= j; rows above hold R) for tile_form_q.  Same steps as
-// my_hou_kernel<128,32> (util/inc/kernelQR.h:215-414): u = x/||x||,
-// u0 += sign(u0), u scaled to ||u||^2 = 2.
-// Look-ahead: once reflector j is in shared memory, the owner of column j+1
-// (another warp) applies it to that column alone, builds reflector j+1 and
-// publishes it (bar.arrive on a named barrier), and only then applies j to its
-// other columns; every other warp waits on that barrier (bar.sync) and applies
-// j to its columns.  The dependency chain per column is then one single-column
-// update and one reflector, not a reflector plus a four-column update and a
-// CTA barrier.  Barrier of column j: 1 + (j & 3) (0 is __syncthreads); at most
-// two are in flight, because a warp must wait on column j before it can
-// publish j + 1.
+// warp w owns columns w, w + 8, w + 16, w + 24, eight lanes per column (lane
+// group q = lane / 8 has column 8 q + w), and lane g of a group the 16 rows
+// 16 (e / 2) + 2 g + e % 2.  Writes R (32 x 32, upper; diag = -sign(x0) ||x||)
+// to Rdst and leaves the reflectors in the tile (column j, zero above row j).
+// Same steps as my_hou_kernel<128,32> (util/inc/kernelQR.h:215-414):
+// u = x/||x||, u0 += sign(u0), u scaled to ||u||^2 = 2.
+//
+// What bounds it: the chain of 32 columns.  Step j starts from the bare column
+// x in shared memory, and x^T a_c of every column and ||x||^2 (each group its
+// own copy) are reduced together; u^T a_c = s x^T a_c follows from the norm, so
+// a column costs one reduction, two reciprocal roots and one CTA barrier, where
+// a dot product with the finished reflector and then the norm took two
+// reductions in a row.  Branches are per warp (lane-wise ones cost more than
+// the work they skip); four warps with four lanes per column were slower.
 struct TileSmem {
-  double V[kNB * kTile];  // reflector j at V[j * kTile ..]
+  __align__(16) double x[2][kTile];  // column j below row j (zero elsewhere)
+  double x0[2];                      // its row j
   double RR[kNB];
 };
-constexpr size_t kTileSmem = sizeof(TileSmem);
 
-__device__ __forceinline__ int qr_bar(int j) { return 1 + (j & 3); }
-__device__ __forceinline__ void qr_bar_arrive(int id) {
-  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "n"(kThreads) : "memory");
-}
-__device__ __forceinline__ void qr_bar_wait(int id) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(kThreads) : "memory");
-}
-
-// Reflector of column j from a[c] (c = j / 8, this warp owns j): writes
-// V[j], RR[j] and the reflector into a[c] (rows >= j).
-__device__ __forceinline__ void tile_reflector(double (&a)[4][kRPL], int j, int mm, int lane,
-                                               TileSmem& sm) {
-  const int oc = j >> 3;
-  double x[kRPL], ss = 0.0;
+// Sums over groups of eight lanes, two at a time.
+__device__ __forceinline__ void sum8x2(double& u, double& v) {
 #pragma unroll
-  for (int i = 0; i < kRPL; ++i) {
-    const int row = lane + 32 * i;
-    double v = 0.0;
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-      if (c == oc) v = a[c][i];
-    x[i] = (row >= j && row < mm) ? v : 0.0;
-    ss = fma(x[i], x[i], ss);
-  }
-  const double nrm2 = warp_sum(ss);
-  const double x0 = __shfl_sync(0xffffffffu, x[0], j);  // row j: lane j, i = 0
-  // A zero column (nothing to annihilate) gets u = sqrt(2) e_j rather than
-  // u = 0: H = I - u u^T then only flips row j, R_jj = 0, every reflector
-  // keeps ||u||^2 = 2, and I - Q stays nonsingular for the Householder
-  // reconstruction (u = 0 would give a zero pivot there).
-  const bool live = nrm2 > 0.0;
-  const double rn = live ? rsqrt(nrm2) : 0.0;  // 1 / ||x||
-  const double u0 = x0 * rn;
-  const double u0n = live ? u0 + ((u0 >= 0.0) ? 1.0 : -1.0) : 1.4142135623730951;
-  const double s2 = live ? rsqrt(fabs(u0n)) : 1.0;
-  if (lane == 0) sm.RR[j] = live ? ((u0 >= 0.0) ? -(nrm2 * rn) : nrm2 * rn) : 0.0;
-#pragma unroll
-  for (int i = 0; i < kRPL; ++i) {
-    const int row = lane + 32 * i;
-    const double u = ((row == j) ? u0n : x[i] * rn) * s2;
-    sm.V[j * kTile + row] = u;
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-      if (c == oc && row >= j) a[c][i] = u;
+  for (int m = 4; m > 0; m >>= 1) {
+    const double a = __shfl_xor_sync(0xffffffffu, u, m);
+    const double b = __shfl_xor_sync(0xffffffffu, v, m);
+    u += a;
+    v += b;
   }
 }
-
 __device__ void tile_factor(double* src, long ld, int mm, double* Rdst, long ldR, TileSmem& sm) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double a[4][kRPL];
+  const int g = lane & 7, col = 8 * (lane >> 3) + warp;
+  constexpr int kE = kTile / 8;  // rows per lane
+  constexpr int kTop = kNB / 8;  // of them in the first 32 rows
+  auto row_of = [&](int e) { return 16 * (e >> 1) + 2 * g + (e & 1); };
+  double a[kE];
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int i = 0; i < kRPL; ++i) {
-      const int row = lane + 32 * i;
-      a[c][i] = (row < mm) ? __ldcg(src + row + (long)(8 * c + warp) * ld) : 0.0;
-    }
+  for (int e = 0; e < kE; ++e)
+    a[e] = (row_of(e) < mm) ? __ldcg(src + row_of(e) + (long)col * ld) : 0.0;
 
-  if (warp == 0) {
-    tile_reflector(a, 0, mm, lane, sm);
-    qr_bar_arrive(qr_bar(0));
-  }
-  for (int j = 0; j < kNB; ++j) {
-    if (warp != (j & 7)) qr_bar_wait(qr_bar(j));  // reflector j is in V[j]
-    double uv[kRPL];
+  // column j to shared memory by the eight lanes that own it
+  auto publish = [&](int j) {
+    double2* x = reinterpret_cast<double2*>(sm.x[j & 1]);
 #pragma unroll
-    for (int i = 0; i < kRPL; ++i) uv[i] = sm.V[j * kTile + lane + 32 * i];
-    const int j1 = j + 1;
-    const bool own1 = j1 < kNB && warp == (j1 & 7);
-    if (own1) {
-      // column j + 1 first, then its reflector, published at once
-      const int c1 = j1 >> 3;
-      double p0 = 0.0, p1 = 0.0;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (c == c1) {
-#pragma unroll
-          for (int i = 0; i < kRPL; i += 2) {
-            p0 = fma(uv[i], a[c][i], p0);
-            p1 = fma(uv[i + 1], a[c][i + 1], p1);
-          }
-        }
-      const double dot = warp_sum(p0 + p1);
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (c == c1) {
-#pragma unroll
-          for (int i = 0; i < kRPL; ++i) a[c][i] = fma(-dot, uv[i], a[c][i]);
-        }
-      tile_reflector(a, j1, mm, lane, sm);
-      qr_bar_arrive(qr_bar(j1));
-    }
-    if (8 * 3 + warp <= j) continue;  // all columns of this warp factored (warp-uniform)
-    // the warp's other columns right of j (column j + 1 is done above); the
-    // four dot products are reduced together
-    double pc[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      double p0 = 0.0, p1 = 0.0;
-#pragma unroll
-      for (int i = 0; i < kRPL; i += 2) {
-        p0 = fma(uv[i], a[c][i], p0);
-        p1 = fma(uv[i + 1], a[c][i + 1], p1);
+    for (int e = 0; e < kE; e += 2) {
+      const int row = row_of(e);  // rows of e >= kTop are all below row j
+      x[row >> 1] = make_double2(e >= kTop || row > j ? a[e] : 0.0,
+                                 e >= kTop || row + 1 > j ? a[e + 1] : 0.0);
+      if (e < kTop) {
+        if (row == j) sm.x0[j & 1] = a[e];
+        if (row + 1 == j) sm.x0[j & 1] = a[e + 1];
       }
-      pc[c] = p0 + p1;
     }
-    warp_sum4(pc, lane);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int h = 8 * c + warp;
-      const double dot = (h > j && h != j1) ? pc[c] : 0.0;
-#pragma unroll
-      for (int i = 0; i < kRPL; ++i) a[c][i] = fma(-dot, uv[i], a[c][i]);
-    }
-  }
-  __syncthreads();  // RR complete
-
-  // R: row k = lane (i = 0), column h = 8c + w; reflectors back into the tile
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int h = 8 * c + warp;
-    const double r = (lane < h) ? a[c][0] : ((lane == h) ? sm.RR[h] : 0.0);
-    Rdst[lane + (long)h * ldR] = r;
-#pragma unroll
-    for (int i = 0; i < kRPL; ++i) {
-      const int row = lane + 32 * i;
-      if (row < mm) src[row + (long)h * ld] = a[c][i];
-    }
-  }
-}
-
-// Explicit thin Q = H_0 ... H_31 I[:, :32] of a factored tile, from the
-// reflectors left in it, accumulated backwards and written over them.  Before
-// H_j is applied, columns c < j are still e_c, which H_j leaves unchanged, so
-// warps whose columns are all left of j skip the step.
-__device__ void tile_form_q(double* src, long ld, int mm, TileSmem& sm, double* qtop_copy) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int e = threadIdx.x; e < kNB * kTile; e += kThreads) {
-    const int j = e / kTile, row = e % kTile;
-    sm.V[e] = (row >= j && row < mm) ? __ldcg(src + row + (long)j * ld) : 0.0;
-  }
+  };
+  if (col == 0) publish(0);
   __syncthreads();
-  double q[4][kRPL];
+#pragma unroll 1
+  for (int j = 0; j < kNB; ++j) {
+    double x[kE], d0 = 0.0, d1 = 0.0, n0 = 0.0, n1 = 0.0;
+    const double2* xs = reinterpret_cast<const double2*>(sm.x[j & 1]);
+    const double x0 = sm.x0[j & 1];
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int i = 0; i < kRPL; ++i) q[c][i] = (lane + 32 * i == 4 * warp + c) ? 1.0 : 0.0;
-  for (int j = kNB - 1; j >= 0; --j) {
-    if (4 * warp + 3 < j) continue;  // warp-uniform
-    double uv[kRPL];
-#pragma unroll
-    for (int i = 0; i < kRPL; ++i) uv[i] = sm.V[j * kTile + lane + 32 * i];
-    double pc[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      double p0 = 0.0, p1 = 0.0;
-#pragma unroll
-      for (int i = 0; i < kRPL; i += 2) {
-        p0 = fma(uv[i], q[c][i], p0);
-        p1 = fma(uv[i + 1], q[c][i + 1], p1);
-      }
-      pc[c] = p0 + p1;
+    for (int e = 0; e < kE; e += 2) {
+      const double2 v = xs[row_of(e) >> 1];
+      x[e] = v.x;
+      x[e + 1] = v.y;
+      n0 = fma(v.x, v.x, n0);
+      n1 = fma(v.y, v.y, n1);
+      d0 = fma(v.x, a[e], d0);
+      d1 = fma(v.y, a[e + 1], d1);
     }
-    warp_sum4(pc, lane);
+    // this column's row j: lane (j / 2) % 8 of the group, e = 2 (j / 16) + j % 2
+    const double e0 = (j & 1) ? a[1] : a[0], e1 = (j & 1) ? a[3] : a[2];
+    const double aj = __shfl_sync(0xffffffffu, (j & 16) ? e1 : e0, (lane & 24) | ((j >> 1) & 7));
+    double nrm2 = n0 + n1, dot = d0 + d1;
+    sum8x2(nrm2, dot);
+    nrm2 = fma(x0, x0, nrm2);
+    // A zero column (nothing to annihilate) gets u = sqrt(2) e_j rather than
+    // u = 0: H = I - u u^T then only flips row j, R_jj = 0, every reflector
+    // keeps ||u||^2 = 2, and I - Q stays nonsingular for the Householder
+    // reconstruction (u = 0 would give a zero pivot there).
+    const bool live = nrm2 > 0.0;
+    const double rn = live ? rsqrt(nrm2) : 0.0;  // 1 / ||x||
+    const double c0 = x0 * rn;
+    const double sg = (c0 >= 0.0) ? 1.0 : -1.0;
+    const double c0n = c0 + sg;
+    const double s2 = rsqrt(fabs(c0n));
+    const double sc = rn * s2;                               // u = sc x below row j
+    const double u0 = live ? c0n * s2 : 1.4142135623730951;  // u in row j
+    const double d = (col > j) ? fma(sc, dot, u0 * aj) : 0.0;  // u^T a
+    const double f = -d * sc, fj = -d * u0;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double dot = (4 * warp + c >= j) ? pc[c] : 0.0;
+    for (int e = 0; e < kTop; ++e) a[e] += (row_of(e) == j) ? fj : 0.0;
 #pragma unroll
-      for (int i = 0; i < kRPL; ++i) q[c][i] = fma(-dot, uv[i], q[c][i]);
+    for (int e = 0; e < kE; ++e) a[e] = fma(f, x[e], a[e]);
+    if (warp == ((j + 1) & 7) && j + 1 < kNB) {
+      if (col == j + 1) publish(j + 1);
     }
+    if (warp == (j & 7)) {  // column j itself: its reflector
+      const bool mine = col == j;
+#pragma unroll
+      for (int e = 0; e < kE; ++e)
+        a[e] = (mine && (e >= kTop || row_of(e) > j)) ? sc * x[e] : a[e];
+#pragma unroll
+      for (int e = 0; e < kTop; ++e) a[e] = (mine && row_of(e) == j) ? u0 : a[e];
+      if (lane == 0) sm.RR[j] = -sg * (nrm2 * rn);
+    }
+    __syncthreads();
   }
+
+  // R from the rows above the diagonal; reflectors back into the tile
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int i = 0; i < kRPL; ++i) {
-      const int row = lane + 32 * i;
-      if (row < mm) {
-        src[row + (long)(4 * warp + c) * ld] = q[c][i];
-        if (qtop_copy && row < kNB) qtop_copy[row + (4 * warp + c) * kNB] = q[c][i];
-      }
+  for (int e = 0; e < kE; ++e) {
+    const int row = row_of(e);
+    if (e < kTop) {
+      Rdst[row + (long)col * ldR] = (row < col) ? a[e] : ((row == col) ? sm.RR[col] : 0.0);
+      if (row < col) a[e] = 0.0;
     }
+    if (row < mm) src[row + (long)col * ld] = a[e];
+  }
 }
 
 __global__ void __launch_bounds__(kThreads, 1) tsqr_up_kernel(const TsqrPlan plan, double* A,
                                                               long lda, double* ws, double* Rout,
                                                               long ldr) {
-  extern __shared__ __align__(16) double up_smem[];
-  TileSmem& sm = *reinterpret_cast<TileSmem*>(up_smem);
+  __shared__ TileSmem sm;
   __shared__ int is_last;
   int* cnt = reinterpret_cast<int*>(ws + plan.cnt_off);
   int level = 0, idx = blockIdx.x;
@@ -359,78 +260,219 @@ __global__ void __launch_bounds__(kThreads, 1) tsqr_up_kernel(const TsqrPlan pla
   }
 }
 
+// ---- 32-wide products on the FP64 tensor pipe ----
+// mma.m8n8k4: lane (g, t) = (lane / 4, lane % 4) holds A[g][t], B[t][g] and
+// D[g][2t], D[g][2t+1].  32 x 32 matrices are row-major with kLd doubles per
+// row, 128-row tiles column-major with kVLd per column: both strides are 32
+// bytes mod 128, which makes every fragment read conflict-free.
+constexpr int kLd = 36, kVLd = kTile + 4;
+
+__device__ __forceinline__ void mma8(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+// rows 8 mi .. 8 mi + 7 of A B, all 32 columns of B (both 32 x 32)
+__device__ __forceinline__ void row_block(const double* A, const double* B, int mi,
+                                          double (&d)[4][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int ni = 0; ni < 4; ++ni) d[ni][0] = d[ni][1] = 0.0;
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    const double af = A[(8 * mi + g) * kLd + 4 * kk + t];
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) mma8(d[ni], af, B[(4 * kk + t) * kLd + 8 * ni + g]);
+  }
+}
+
+struct QSmem {
+  double V[kNB * kVLd];
+  double G[kNB * kLd];  // G[j * kLd + i] = (V^T V)_ij, i < j
+  double K[kNB * kLd];
+};
+
+// x[i] -= row[i] * f, i < j, the row read two at a time before the products.
+template <int J>
+__device__ __forceinline__ void eliminate(double (&x)[kNB], const double* row, double f) {
+  double2 t[(J + 1) / 2 + 1];
+#pragma unroll
+  for (int i = 0; i < (J + 1) / 2; ++i) t[i] = *reinterpret_cast<const double2*>(row + 2 * i);
+#pragma unroll
+  for (int i = 0; i < J; ++i) x[i] = fma(-((i & 1) ? t[i / 2].y : t[i / 2].x), f, x[i]);
+}
+// Back substitution, lane = right-hand side: B x = rhs, B upper triangular with
+// B_ij at Bt[j * kLd + i] (i < j) and diagonal 1 / rd (unit when rd is null).
+template <int J = kNB - 1>
+__device__ __forceinline__ void back_solve(double (&x)[kNB], const double* Bt, const double* rd) {
+  if (rd) x[J] *= rd[J];
+  if constexpr (J > 0) {
+    eliminate<J>(x, Bt + J * kLd, x[J]);
+    back_solve<J - 1>(x, Bt, rd);
+  }
+}
+
 // Explicit Q of every tree node, all levels at once (the up-sweep left the
-// reflectors in each node's tile): one CTA per node.
-__global__ void __launch_bounds__(kThreads, 1) tsqr_q_kernel(const TsqrPlan plan, double* A,
-                                                             long lda, double* ws) {
+// reflectors in each node's tile): one CTA per node, Q = E - V K.
+__global__ void __launch_bounds__(kThreads, 1)
+    tsqr_q_kernel(const TsqrPlan plan, double* A, long lda, double* ws) {
   extern __shared__ __align__(16) double q_smem[];
-  TileSmem& sm = *reinterpret_cast<TileSmem*>(q_smem);
+  QSmem& sm = *reinterpret_cast<QSmem*>(q_smem);
   int idx = blockIdx.x, level = 0;
   while (level < plan.nlev && idx >= plan.T[level]) {
     idx -= plan.T[level];
     ++level;
   }
   if (level >= plan.nlev) return;
-  double* src;
-  long ld;
-  if (level == 0) {
-    src = A + (long)idx * kTile;
-    ld = lda;
-  } else {
-    src = ws + plan.soff[level] + (long)idx * kTile;
-    ld = plan.rows[level];
-  }
+  double* src = (level == 0) ? A + (long)idx * kTile : ws + plan.soff[level] + (long)idx * kTile;
+  const long ld = (level == 0) ? lda : plan.rows[level];
   const int mm = min(kTile, plan.rows[level] - idx * kTile);
-  tile_form_q(src, ld, mm, sm, (level == 0 && idx == 0) ? ws + plan.qtop_off : nullptr);
-}
-
-struct FinishSmem {
-  double M[kNB * (kNB + 1)];
-  double T[kNB * (kNB + 1)];
-  double B[kNB * (kNB + 1)];
-  double LU[kNB * (kNB + 1)];
-};
-
-// C = Bm * M (32x32x32) into Out (all padded stride 33), 256 threads.
-__device__ void mul32(const double* Bm, const double* M, double* Out) {
-  for (int e = threadIdx.x; e < kNB * kNB; e += kThreads) {
-    int r = e & 31, c = e >> 5;
-    double s = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < kNB; ++k) s = fma(Bm[r * 33 + k], M[k * 33 + c], s);
-    Out[r * 33 + c] = s;
-  }
-}
-
-// Path product for leaf tile t: M = B_1 (B_2 (... B_top)) with
-// B_L = S_L[32*idx_{L-1} : +32, :].  Result in sm.M.
-__device__ void path_product(const TsqrPlan& plan, const double* ws, int t, FinishSmem& sm) {
-  int idxs[kMaxLevels];
-  idxs[0] = t;
-  for (int L = 1; L < plan.nlev; ++L) idxs[L] = idxs[L - 1] / kFan;
-  for (int e = threadIdx.x; e < kNB * kNB; e += kThreads) {
-    int r = e & 31, c = e >> 5;
-    sm.M[r * 33 + c] = (r == c) ? 1.0 : 0.0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int e = threadIdx.x; e < kNB * kTile; e += kThreads) {
+    const int j = e / kTile, row = e % kTile;
+    sm.V[j * kVLd + row] = (row < mm) ? __ldcg(src + row + (long)j * ld) : 0.0;
   }
   __syncthreads();
-  for (int L = plan.nlev - 1; L >= 1; --L) {
-    const double* S = ws + plan.soff[L];
-    long ld = plan.rows[L];
-    long r0 = (long)kNB * idxs[L - 1];
-    for (int e = threadIdx.x; e < kNB * kNB; e += kThreads) {
-      int r = e & 31, c = e >> 5;
-      sm.B[r * 33 + c] = __ldcg(S + r0 + r + (long)c * ld);
+  // the ten upper 8 x 8 tiles of V^T V
+  for (int q = warp; q < 10; q += kThreads / 32) {
+    const int nj = (q < 1) ? 0 : (q < 3) ? 1 : (q < 6) ? 2 : 3;
+    const int mi = q - nj * (nj + 1) / 2;
+    double d[2] = {0.0, 0.0}, f[2] = {0.0, 0.0};
+    const double* va = sm.V + (8 * mi + g) * kVLd + t;
+    const double* vb = sm.V + (8 * nj + g) * kVLd + t;
+#pragma unroll 8
+    for (int kk = 0; kk < kTile / 8; ++kk) {
+      mma8(d, va[8 * kk], vb[8 * kk]);
+      mma8(f, va[8 * kk + 4], vb[8 * kk + 4]);
     }
-    __syncthreads();
-    mul32(sm.B, sm.M, sm.T);
-    __syncthreads();
-    for (int e = threadIdx.x; e < kNB * kNB; e += kThreads) {
-      int r = e & 31, c = e >> 5;
-      sm.M[r * 33 + c] = sm.T[r * 33 + c];
+    sm.G[(8 * nj + 2 * t) * kLd + 8 * mi + g] = d[0] + f[0];
+    sm.G[(8 * nj + 2 * t + 1) * kLd + 8 * mi + g] = d[1] + f[1];
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // (I + striu(G)) K = V_top^T, column `lane` of K
+    double k[kNB];
+#pragma unroll
+    for (int i = 0; i < kNB; ++i) k[i] = sm.V[i * kVLd + lane];
+    back_solve(k, sm.G, nullptr);
+#pragma unroll
+    for (int i = 0; i < kNB; ++i) sm.K[i * kLd + lane] = k[i];
+  }
+  __syncthreads();
+  for (int mi = warp; mi < kTile / 8; mi += kThreads / 32) {
+    double d[4][2];
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) d[ni][0] = d[ni][1] = 0.0;
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      const double af = sm.V[(4 * kk + t) * kVLd + 8 * mi + g];
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) mma8(d[ni], af, sm.K[(4 * kk + t) * kLd + 8 * ni + g]);
     }
-    __syncthreads();
+    const int row = 8 * mi + g;
+    if (row >= mm) continue;
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = 8 * ni + 2 * t + h;
+        const double v = ((row == c) ? 1.0 : 0.0) - d[ni][h];
+        src[row + (long)c * ld] = v;
+        // leaf 0's tile is overwritten by the finishing kernel's CTA 0
+        if (blockIdx.x == 0 && row < kNB) ws[plan.qtop_off + row * kNB + c] = v;
+      }
   }
 }
+
+constexpr int kHalf = kThreads / 2;  // threads of a group of the finishing kernel
+
+struct FinishSmem {
+  double Q[kNB * kVLd];  // this CTA's rows of its leaf's Q
+  // per group (0: this CTA's leaf, 1: leaf 0): the current block, two products
+  double B[2][kNB * kLd], M[2][2][kNB * kLd];
+  double Ui[kNB * kLd];  // U^{-1}
+  double Li[kNB * kLd];  // L1^{-T}
+  double L[kNB * kLd];   // L1, row-major: L1^T by columns
+  double Ut[kNB * kLd];  // U by columns
+  double rd[kNB];        // 1 / U_jj
+  double A0[kNB * kLd];  // (I - Q)[0:32]
+};
+
+// 1 / x of a normal number to about an ulp: the hardware's approximation and two
+// Newton steps, without the branches of a division.
+__device__ __forceinline__ double reciprocal(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(r, fma(-x, r, 1.0), r);
+  return fma(r, fma(-x, r, 1.0), r);
+}
+
+__device__ __forceinline__ void group_bar(int grp) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kHalf) : "memory");
+}
+// Out = s * A B + (ident ? I : 0), all 32 x 32, by a group of four warps.
+__device__ __forceinline__ void group_mul(const double* A, const double* B, double* Out, double s,
+                                          bool ident) {
+  const int w = (threadIdx.x & (kHalf - 1)) >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, q = lane & 3;
+  double d[4][2];
+  row_block(A, B, w, d);
+#pragma unroll
+  for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 8 * w + g, c = 8 * ni + 2 * q + h;
+      Out[r * kLd + c] = fma(s, d[ni][h], (ident && r == c) ? 1.0 : 0.0);
+    }
+}
+
+// Path product down the tree to leaf t, M = B_1 (B_2 (... B_top)) with B_L the
+// rows of level L's Q that belong to the child on the path; returns M.
+__device__ const double* walk(const TsqrPlan& plan, const double* __restrict__ ws, int t, int grp,
+                              FinishSmem& sm) {
+  const int tid = threadIdx.x & (kHalf - 1);
+  constexpr int kPer = kNB * kNB / kHalf;  // elements per thread of a 32 x 32 block
+  double br[kPer];
+  auto fetch = [&](int level) {  // level >= 1
+    const double* b = ws + plan.soff[level] + (long)kNB * (t >> (2 * (level - 1)));
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const int at = tid + e * kHalf;
+      br[e] = __ldcg(b + (at & 31) + (long)(at >> 5) * plan.rows[level]);
+    }
+  };
+  auto put = [&](double* dst) {
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const int at = tid + e * kHalf;
+      dst[(at & 31) * kLd + (at >> 5)] = br[e];
+    }
+  };
+  int level = plan.nlev - 1, cur = 0;
+  if (level == 0) {
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const int at = tid + e * kHalf;
+      sm.M[grp][0][(at >> 5) * kLd + (at & 31)] = ((at >> 5) == (at & 31)) ? 1.0 : 0.0;
+    }
+    group_bar(grp);
+    return sm.M[grp][0];
+  }
+  fetch(level);
+  put(sm.M[grp][0]);
+  while (--level > 0) {
+    fetch(level);
+    put(sm.B[grp]);
+    group_bar(grp);
+    group_mul(sm.B[grp], sm.M[grp][cur], sm.M[grp][cur ^ 1], 1.0, false);
+    cur ^= 1;
+    group_bar(grp);
+  }
+  group_bar(grp);
+  return sm.M[grp][cur];
+}
+static_assert(kFan == 4, "walk() shifts the child index by two bits per level");
 
 // mode 0: write the explicit thin Q into A (evd_tsqr).
 // mode 1: write Y (into Yout), W (into Wout), and optionally the band panel
@@ -439,143 +481,133 @@ __global__ void __launch_bounds__(kThreads, 1)
     tsqr_finish_kernel(const TsqrPlan plan, const double* ws, double* A, long lda, int mode,
                        double* Yout, long ldy, double* Wout, long ldw, const double* Rin,
                        long ldr, double* Aband, long ldband) {
-  extern __shared__ double dsm[];
-  __shared__ FinishSmem sm;
-  double* Qs = dsm;                   // 128 x 33 : rows of Q (then Y)
-  double* Ws = dsm + kSub * 33;       // 128 x 33 : W rows
+  extern __shared__ __align__(16) double dsm[];
+  FinishSmem& sm = *reinterpret_cast<FinishSmem*>(dsm);
   const int t = blockIdx.x;
-  const int r0 = t * kSub;
-  const int mm = min(kSub, plan.m - r0);
-  const int leaf = r0 / kTile;       // TSQR leaf tile holding these rows
-
-  // tile rows of Q = Qleaf_t * M_t; the leaf Q tile is staged in shared
-  // memory (coalesced) before the product
-  for (int e = threadIdx.x; e < kSub * kNB; e += kThreads) {
-    int r = e & (kSub - 1), c = e >> 7;
-    Ws[r * 33 + c] = (r < mm) ? __ldcg(A + (long)(r0 + r) + (long)c * lda) : 0.0;
-  }
-  path_product(plan, ws, leaf, sm);  // ends with __syncthreads
-  for (int e = threadIdx.x; e < kSub * kNB; e += kThreads) {
-    int r = e & (kSub - 1), c = e >> 7;
-    double s = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < kNB; ++k) s = fma(Ws[r * 33 + k], sm.M[k * 33 + c], s);
-    Qs[r * 33 + c] = s;
+  const int r0 = t * kTile;
+  const int mm = min(kTile, plan.m - r0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int grp = threadIdx.x / kHalf;
+  const double* M = nullptr;
+  if (grp == 0) {
+#pragma unroll 16
+    for (int e = threadIdx.x; e < kNB * kTile; e += kHalf) {
+      const int j = e / kTile, row = e % kTile;
+      sm.Q[j * kVLd + row] = (row < mm) ? __ldcg(A + (long)(r0 + row) + (long)j * lda) : 0.0;
+    }
+    walk(plan, ws, t, 0, sm);
+  } else if (mode == 1) {
+    M = walk(plan, ws, 0, 1, sm);
+    for (int at = threadIdx.x - kHalf; at < kNB * kNB; at += kHalf)
+      sm.B[1][(at >> 5) * kLd + (at & 31)] = __ldcg(ws + plan.qtop_off + at);
+    group_bar(1);
+    group_mul(sm.B[1], M, sm.A0, -1.0, true);
+    group_bar(1);
+    const int w1 = warp - kHalf / 32;
+    if (w1 == 0) {
+      // unpivoted LU by one warp (lane = row, the row in registers; row k is
+      // broadcast by shuffles, all issued before the pivot's reciprocal is
+      // needed): 14k cycles; a rolled loop, rows through shared memory and four
+      // warps with a barrier per step took 16k to 29k
+      double lu[kNB];
+#pragma unroll
+      for (int c = 0; c < kNB; ++c) lu[c] = sm.A0[lane * kLd + c];
+#pragma unroll
+      for (int k = 0; k < kNB; ++k) {
+        double row[kNB];
+#pragma unroll
+        for (int c = k; c < kNB; ++c) row[c] = __shfl_sync(0xffffffffu, lu[c], k);
+        const double rp = reciprocal(row[k]);
+        if (lane == 0) sm.rd[k] = rp;
+        const double l = (lane > k) ? lu[k] * rp : 0.0;
+        if (lane > k) lu[k] = l;
+#pragma unroll
+        for (int c = k + 1; c < kNB; ++c) lu[c] = fma(-l, row[c], lu[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < kNB; ++c) {
+        sm.L[lane * kLd + c] = (c < lane) ? lu[c] : ((c == lane) ? 1.0 : 0.0);
+        sm.Ut[c * kLd + lane] = (c >= lane) ? lu[c] : 0.0;
+      }
+    }
+    group_bar(1);
+    // both inverses, lane = column
+    if (w1 < 2) {
+      double x[kNB];
+#pragma unroll
+      for (int i = 0; i < kNB; ++i) x[i] = (i == lane) ? 1.0 : 0.0;
+      if (w1 == 0) back_solve(x, sm.Ut, sm.rd);
+      else back_solve(x, sm.L, nullptr);
+      double* dst = (w1 == 0) ? sm.Ui : sm.Li;
+#pragma unroll
+      for (int i = 0; i < kNB; ++i) dst[i * kLd + lane] = x[i];
+    }
   }
   __syncthreads();
+  M = sm.M[0][max(plan.nlev - 2, 0) & 1];  // where walk() left this leaf's product
 
   if (mode == 0) {
-    for (int e = threadIdx.x; e < kSub * kNB; e += kThreads) {
-      int r = e & (kSub - 1), c = e >> 7;
-      if (r < mm) A[(long)(r0 + r) + (long)c * lda] = Qs[r * 33 + c];
+    for (int mi = warp; mi < kTile / 8; mi += kThreads / 32) {
+      double d[4][2];
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) d[ni][0] = d[ni][1] = 0.0;
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        const double af = sm.Q[(4 * kk + q) * kVLd + 8 * mi + g];
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) mma8(d[ni], af, M[(4 * kk + q) * kLd + 8 * ni + g]);
+      }
+      const int row = 8 * mi + g;
+      if (row >= mm) continue;
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) A[(long)(r0 + row) + (long)(8 * ni + 2 * q + h) * lda] = d[ni][h];
     }
     return;
   }
 
-  // LU of (I - Qtop), Qtop = Qleaf_0[0:32] * M_0 (recomputed by every CTA)
-  if (leaf != 0) path_product(plan, ws, 0, sm);
-  {
-    const double* q0 = ws + plan.qtop_off;
-    if (t == 0) {
-      for (int e = threadIdx.x; e < kNB * kNB; e += kThreads) {
-        int r = e & 31, c = e >> 5;
-        sm.LU[r * 33 + c] = ((r == c) ? 1.0 : 0.0) - Qs[r * 33 + c];
-      }
-    } else {
-      for (int e = threadIdx.x; e < kNB * kNB; e += kThreads) {
-        int r = e & 31, c = e >> 5;
-        double s = 0.0;
-#pragma unroll 8
-        for (int k = 0; k < kNB; ++k) s = fma(__ldcg(q0 + r + k * kNB), sm.M[k * 33 + c], s);
-        sm.LU[r * 33 + c] = ((r == c) ? 1.0 : 0.0) - s;
+  // rows >= 32: I - Q = -Q_leaf M, so Y = -Q_leaf (M U^{-1}), W = -Q_leaf (M L1^{-T});
+  // the products (negated) go to B[0] and B[1]
+  group_mul(M, grp ? sm.Li : sm.Ui, sm.B[grp], -1.0, false);
+  __syncthreads();
+  for (int mi = warp; mi < kTile / 8; mi += kThreads / 32) {
+    const bool head = t == 0 && mi < kNB / 8;
+    const double* by = head ? sm.Ui : sm.B[0];
+    const double* bw = head ? sm.Li : sm.B[1];
+    double y[4][2], z[4][2];
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) y[ni][0] = y[ni][1] = z[ni][0] = z[ni][1] = 0.0;
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      const double af = head ? sm.A0[(8 * mi + g) * kLd + 4 * kk + q]
+                             : sm.Q[(4 * kk + q) * kVLd + 8 * mi + g];
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) {
+        mma8(y[ni], af, by[(4 * kk + q) * kLd + 8 * ni + g]);
+        mma8(z[ni], af, bw[(4 * kk + q) * kLd + 8 * ni + g]);
       }
     }
-  }
-  __syncthreads();
-  // unpivoted LU in place (one warp, lane = row, the row in registers; row k
-  // is broadcast by shuffles)
-  if (threadIdx.x < 32) {
-    const int r = threadIdx.x;
-    double lu[kNB];
+    const int row = 8 * mi + g;
+    if (row >= mm) continue;
+    const long gr = r0 + row;
 #pragma unroll
-    for (int c = 0; c < kNB; ++c) lu[c] = sm.LU[r * 33 + c];
+    for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-    for (int k = 0; k < kNB; ++k) {
-      const double piv = __shfl_sync(0xffffffffu, lu[k], k);
-      const double l = lu[k] / piv;
-      if (r > k) lu[k] = l;
-#pragma unroll
-      for (int c = k + 1; c < kNB; ++c) {
-        const double ukc = __shfl_sync(0xffffffffu, lu[c], k);
-        if (r > k) lu[c] = fma(-l, ukc, lu[c]);
+      for (int h = 0; h < 2; ++h) {
+        const int c = 8 * ni + 2 * q + h;
+        Yout[gr + (long)c * ldy] = head ? sm.L[row * kLd + c] : y[ni][h];
+        Wout[gr + (long)c * ldw] = z[ni][h];
+        if (Aband)
+          Aband[gr + (long)c * ldband] =
+              (gr < kNB && c >= gr) ? __ldcg(Rin + gr + (long)c * ldr) : 0.0;
       }
-    }
-#pragma unroll
-    for (int c = 0; c < kNB; ++c) sm.LU[r * 33 + c] = lu[c];
-  }
-  __syncthreads();
-
-  // per row: iq = e_gr - q ;  even thread -> Y row, odd thread -> W row
-  const int row = threadIdx.x >> 1;
-  const bool doW = threadIdx.x & 1;
-  double x[kNB];
-  if (row < mm) {
-    const int gr = r0 + row;
-#pragma unroll
-    for (int h = 0; h < kNB; ++h) x[h] = ((gr == h) ? 1.0 : 0.0) - Qs[row * 33 + h];
-    if (!doW) {
-      if (gr < kNB) {
-#pragma unroll
-        for (int h = 0; h < kNB; ++h) x[h] = (h < gr) ? sm.LU[gr * 33 + h] : ((h == gr) ? 1.0 : 0.0);
-      } else {
-        // y U = iq  (U upper, non-unit)
-#pragma unroll
-        for (int h = 0; h < kNB; ++h) {
-          double s = x[h];
-#pragma unroll
-          for (int k = 0; k < h; ++k) s = fma(-x[k], sm.LU[k * 33 + h], s);
-          x[h] = s / sm.LU[h * 33 + h];
-        }
-      }
-    } else {
-      // w L1^T = iq  (L1 unit lower): w_j = iq_j - sum_{k<j} L1[j,k] w_k
-#pragma unroll
-      for (int h = 0; h < kNB; ++h) {
-        double s = x[h];
-#pragma unroll
-        for (int k = 0; k < h; ++k) s = fma(-sm.LU[h * 33 + k], x[k], s);
-        x[h] = s;
-      }
-    }
-  }
-  __syncthreads();
-  if (row < mm) {
-    double* dst = doW ? Ws : Qs;
-#pragma unroll
-    for (int h = 0; h < kNB; ++h) dst[row * 33 + h] = x[h];
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < kSub * kNB; e += kThreads) {
-    int r = e & (kSub - 1), c = e >> 7;
-    if (r < mm) {
-      long gr = r0 + r;
-      Yout[gr + (long)c * ldy] = Qs[r * 33 + c];
-      Wout[gr + (long)c * ldw] = Ws[r * 33 + c];
-      if (Aband) {
-        double v = 0.0;
-        if (gr < kNB && c >= gr) v = __ldcg(Rin + gr + (long)c * ldr);
-        Aband[gr + (long)c * ldband] = v;
-      }
-    }
   }
 }
 
-constexpr size_t kFinishDyn = 2 * kSub * 33 * sizeof(double);
-
 int finish_attr() {
-  EVD_TRY(smem_attr_once((const void*)tsqr_finish_kernel, (int)kFinishDyn));
-  EVD_TRY(smem_attr_once((const void*)tsqr_up_kernel, (int)kTileSmem));
-  EVD_TRY(smem_attr_once((const void*)tsqr_q_kernel, (int)kTileSmem));
+  EVD_TRY(smem_attr_once((const void*)tsqr_finish_kernel, (int)sizeof(FinishSmem)));
+  EVD_TRY(smem_attr_once((const void*)tsqr_q_kernel, (int)sizeof(QSmem)));
   return EVD_SUCCESS;
 }
 
@@ -596,19 +628,24 @@ int panel_counters_reset(long m, double* ws, cudaStream_t st) {
   return EVD_SUCCESS;
 }
 
+// Three launches.  Measured on B200, us per panel, before (explicit node Q's by
+// 32 rank-1 updates, dot products after finished reflectors, row-by-row solves)
+// -> now: m = 128 89 -> 47, 992 178 -> 93, 4096 235 -> 119, 16384 226 -> 148.
+// What is left: 21 us per tree level (32 dependent columns), then 6 us for the
+// node Q's and 16 us to finish, half of it the 32 steps of the LU.
 int panel_qr_launch(long m, double* A, long lda, double* ws, int mode, double* Yout, long ldy,
                     double* Wout, long ldw, double* R, long ldr, double* Aband, long ldband,
                     cudaStream_t st) {
   TsqrPlan plan = make_plan(m);
   if (plan.nlev >= kMaxLevels) return EVD_ERR_INVALID_ARG;
   EVD_TRY(finish_attr());
-  tsqr_up_kernel<<<plan.T[0], kThreads, kTileSmem, st>>>(plan, A, lda, ws, R, ldr);
+  tsqr_up_kernel<<<plan.T[0], kThreads, 0, st>>>(plan, A, lda, ws, R, ldr);
   EVD_LAUNCHED();
   int nodes = 0;
   for (int l = 0; l < plan.nlev; ++l) nodes += plan.T[l];
-  tsqr_q_kernel<<<nodes, kThreads, kTileSmem, st>>>(plan, A, lda, ws);
+  tsqr_q_kernel<<<nodes, kThreads, sizeof(QSmem), st>>>(plan, A, lda, ws);
   EVD_LAUNCHED();
-  tsqr_finish_kernel<<<ceil_div_i(m, kSub), kThreads, kFinishDyn, st>>>(
+  tsqr_finish_kernel<<<plan.T[0], kThreads, sizeof(FinishSmem), st>>>(
       plan, ws, A, lda, mode, Yout, ldy, Wout, ldw, R, ldr, Aband, ldband);
   EVD_LAUNCHED();
   return EVD_SUCCESS;
