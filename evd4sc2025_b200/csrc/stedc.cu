@@ -158,90 +158,106 @@ __global__ void init_kernel(long n, long np, int s, const double* d, const doubl
 
 __device__ __forceinline__ double sign_of(double a, double b) { return (b >= 0.0) ? fabs(a) : -fabs(a); }
 
-// One warp per leaf; lane r owns row r of the leaf eigenvector matrix.
-__global__ void leaf_ql_kernel(int s, int nleaves, double* dw, const double* ew, double* Zw,
-                               long ldz, int* err) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= nleaves) return;
-  const long lo = (long)warp * s;
-  double d[kLeafMax], e[kLeafMax], z[kLeafMax];
-  for (int i = 0; i < s; ++i) {
-    d[i] = dw[lo + i];
-    e[i] = (i < s - 1) ? ew[lo + i] : 0.0;
-    z[i] = (i == lane) ? 1.0 : 0.0;
-  }
+// One warp per leaf: lane i holds d_i and e_i, every lane runs the scalar
+// recurrence on values broadcast by shuffles and applies the rotations to its
+// own row of the eigenvector matrix, which stands in shared memory (column c
+// of lane's row at z[c * 32 + lane]: no bank conflicts, no other lane's data).
+// What bounds it: the chain of the rotations, one reciprocal root and about ten
+// products each; hypot and two divisions per rotation and arrays in local
+// memory took 0.48 ms per solve at n = 1000 and 0.45 ms at n = 100.
+constexpr int kLeafWarps = 4;
+__global__ void __launch_bounds__(32 * kLeafWarps)
+    leaf_ql_kernel(int s, int nleaves, double* dw, const double* ew, double* Zw, long ldz,
+                   int* err) {
+  __shared__ double zsm[kLeafWarps][kLeafMax * 32];
+  const unsigned all = 0xffffffffu;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int leaf = blockIdx.x * kLeafWarps + w;
+  if (leaf >= nleaves) return;
+  const long lo = (long)leaf * s;
+  double* z = zsm[w] + lane;
+  for (int c = 0; c < s; ++c) z[c * 32] = (c == lane) ? 1.0 : 0.0;
+  double d = (lane < s) ? dw[lo + lane] : 0.0;
+  double e = (lane < s - 1) ? ew[lo + lane] : 0.0;
   bool fail = false;
   for (int l = 0; l < s && !fail; ++l) {
     int iter = 0;
     for (;;) {
-      int m = l;
-      while (m < s - 1) {
-        double dd = fabs(d[m]) + fabs(d[m + 1]);
-        if (fabs(e[m]) <= kEps * dd) break;
-        ++m;
-      }
+      // m: the first index >= l whose e is negligible (s - 1 when none is)
+      const double dn = __shfl_down_sync(all, d, 1);
+      const bool small = lane >= s - 1 || fabs(e) <= kEps * (fabs(d) + fabs(dn));
+      const int m = __ffs(__ballot_sync(all, small) & (all << l)) - 1;
       if (m == l) break;
       if (++iter > 60) {
         fail = true;
         break;
       }
-      double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
+      const double dl = __shfl_sync(all, d, l), dl1 = __shfl_sync(all, d, l + 1);
+      const double dm = __shfl_sync(all, d, m), el = __shfl_sync(all, e, l);
+      double g = (dl1 - dl) / (2.0 * el);
       double r = hypot(g, 1.0);
-      g = d[m] - d[l] + e[l] / (g + sign_of(r, g));
+      g = dm - dl + el / (g + sign_of(r, g));
       double sn = 1.0, cs = 1.0, p = 0.0;
       bool underflow = false;
+      double zc = z[m * 32];  // column i + 1 of this row
+      double ei = __shfl_sync(all, e, m - 1);
+      double di = __shfl_sync(all, d, m - 1), di1 = dm;
       for (int i = m - 1; i >= l; --i) {
-        double f = sn * e[i];
-        double bb = cs * e[i];
-        r = hypot(f, g);
-        e[i + 1] = r;
+        const double ein = __shfl_sync(all, e, (i - 1) & 31);
+        const double din = __shfl_sync(all, d, (i - 1) & 31);
+        const double zi = z[i * 32];
+        const double f = sn * ei, bb = cs * ei;
+        const double ff = fma(f, f, g * g);
+        double inv;
+        if (ff > 1e-280) {
+          inv = rsqrt(ff);
+          r = ff * inv;
+        } else {
+          r = hypot(f, g);
+          inv = (r != 0.0) ? 1.0 / r : 0.0;
+        }
+        if (lane == i + 1) e = r;
         if (r == 0.0) {
-          d[i + 1] -= p;
-          e[m] = 0.0;
+          if (lane == i + 1) d -= p;
+          if (lane == m) e = 0.0;
+          z[(i + 1) * 32] = zc;
           underflow = true;
           break;
         }
-        sn = f / r;
-        cs = g / r;
-        g = d[i + 1] - p;
-        r = (d[i] - g) * sn + 2.0 * cs * bb;
+        sn = f * inv;
+        cs = g * inv;
+        g = di1 - p;
+        r = (di - g) * sn + 2.0 * cs * bb;
         p = sn * r;
-        d[i + 1] = g + p;
+        if (lane == i + 1) d = g + p;
         g = cs * r - bb;
-        double t = z[i + 1];
-        z[i + 1] = sn * z[i] + cs * t;
-        z[i] = cs * z[i] - sn * t;
+        z[(i + 1) * 32] = sn * zi + cs * zc;
+        zc = cs * zi - sn * zc;
+        ei = ein;
+        di1 = di;
+        di = din;
       }
       if (underflow) continue;
-      d[l] -= p;
-      e[l] = g;
-      e[m] = 0.0;
+      z[l * 32] = zc;
+      if (lane == l) {
+        d -= p;
+        e = g;
+      }
+      if (lane == m) e = 0.0;
     }
   }
   if (fail && lane == 0) atomicCAS(err, 0, kDevNoConvergence);
-  // selection sort ascending (identical in every lane), permuting z
-  for (int i = 0; i < s - 1; ++i) {
-    int k = i;
-    double v = d[i];
-    for (int j = i + 1; j < s; ++j)
-      if (d[j] < v) {
-        k = j;
-        v = d[j];
-      }
-    if (k != i) {
-      d[k] = d[i];
-      d[i] = v;
-      double t = z[i];
-      z[i] = z[k];
-      z[k] = t;
-    }
+  // ascending order: column c goes to the rank of d_c
+  int rank = 0;
+  for (int c = 0; c < s; ++c) {
+    const double dc = __shfl_sync(all, d, c);
+    rank += (dc < d || (dc == d && c < lane)) ? 1 : 0;
   }
-  if (lane < s) {
-    for (int c = 0; c < s; ++c) Zw[(lo + lane) + (lo + c) * ldz] = z[c];
+  for (int c = 0; c < s; ++c) {
+    const int to = __shfl_sync(all, rank, c);
+    if (lane < s) Zw[(lo + lane) + (lo + to) * ldz] = z[c * 32];
   }
-  if (lane == 0)
-    for (int i = 0; i < s; ++i) dw[lo + i] = d[i];
+  if (lane < s) dw[lo + rank] = d;
 }
 
 // ----------------------------------------------------------------- merges
@@ -257,6 +273,7 @@ struct LevelArgs {
   int* err;
   double *Qt, *Qb, *Ut, *Ub, *Zn;
   int K12max, K23max, Kmax;
+  int chunk;  // columns per CTA of the copy kernels
 };
 
 // z vector, rho and the merged sort order.  grid (ceil(N/256), nm)
@@ -300,20 +317,44 @@ __global__ void merge_setup_kernel(LevelArgs a) {
 
 // Deflation of one merge (LAPACK dlaed2's tests, the reference's host dstedc):
 // small components of z, then Givens pair deflation of neighbours in the merged
-// order.  The pair test chains through the previous undeflated entry, so one
-// thread scans; the block stages the inputs in shared memory chunk by chunk
-// (the scan never waits on global loads), reduces the tolerance in parallel and
-// finishes the type-ordered GEMM positions in parallel.  grid nm, block
-// kDefThreads.
-constexpr int kDefThreads = 256;
-constexpr int kDefChunk = 2048;
+// order.  The pair test of an entry uses the last entry that survived, which is
+// its original neighbour unless a rotation has just changed it.  So all tests
+// run in parallel against the original neighbours; one thread then walks the
+// entries whose test asks for a rotation (and only the runs that those change),
+// and the output positions, in the order of a sequential scan, are prefix
+// counts.  The scan by one thread took 0.35 us per entry, 3 ms of a solve at
+// n = 4096; same decisions and values.  grid nm, a thread per entry of a chunk.
+constexpr int kDefMax = 1024;
 
-__global__ void __launch_bounds__(kDefThreads) merge_deflate_kernel(LevelArgs a) {
-  __shared__ double s_d[kDefChunk], s_z[kDefChunk];
-  __shared__ int s_c[kDefChunk];
-  __shared__ double s_red[2][kDefThreads / 32];
-  __shared__ int s_bad, s_K, s_K1, s_K2;
-  const int m = blockIdx.x;
+// Exclusive prefix of `flag` over the block and its total; two barriers.
+__device__ __forceinline__ int block_prefix(bool flag, int* s_cnt, int* total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const unsigned b = __ballot_sync(0xffffffffu, flag);
+  if (lane == 0) s_cnt[wid] = __popc(b);
+  __syncthreads();
+  int before = 0, sum = 0;
+  for (int w = 0; w < nw; ++w) {
+    const int c = s_cnt[w];
+    before += (w < wid) ? c : 0;
+    sum += c;
+  }
+  __syncthreads();
+  *total = sum;
+  return before + __popc(b & ((1u << lane) - 1u));
+}
+
+__global__ void __launch_bounds__(kDefMax) merge_deflate_kernel(LevelArgs a) {
+  // entry 0 is the survivor pending from the previous chunk, entry 1 + i the
+  // chunk's element i
+  __shared__ double s_d[kDefMax + 1], s_z[kDefMax + 1];
+  __shared__ int s_c[kDefMax + 1], s_prev[kDefMax + 1], s_next[kDefMax + 1];
+  __shared__ signed char s_t[kDefMax + 1], s_rot[kDefMax + 1];
+  __shared__ double s_dp[kDefMax + 1];  // what a rotation at this entry deflates
+  __shared__ double s_red[2][kDefMax / 32];
+  __shared__ int s_cnt[kDefMax / 32];
+  __shared__ unsigned s_cand[kDefMax / 32], s_live[kDefMax / 32];
+  __shared__ int s_nr, s_bad;
+  const int m = blockIdx.x, nthr = blockDim.x, nw = nthr >> 5;
   const long lo = (long)m * a.N;
   const int N = a.N, n1 = a.n1;
   const double rho = a.rho[m];
@@ -322,7 +363,7 @@ __global__ void __launch_bounds__(kDefThreads) merge_deflate_kernel(LevelArgs a)
   const int* perm = a.perm + lo;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   double dmax = 0.0, zmax = 0.0;
-  for (int k = tid; k < N; k += kDefThreads) {
+  for (int k = tid; k < N; k += nthr) {
     dmax = fmax(dmax, fabs(ds[k]));
     zmax = fmax(zmax, fabs(zs[k]));
   }
@@ -332,11 +373,14 @@ __global__ void __launch_bounds__(kDefThreads) merge_deflate_kernel(LevelArgs a)
     s_red[0][wid] = dmax;
     s_red[1][wid] = zmax;
   }
-  if (tid == 0) s_bad = 0;
+  if (tid == 0) {
+    s_bad = 0;
+    s_nr = 0;
+  }
   __syncthreads();
   dmax = 0.0;
   zmax = 0.0;
-  for (int w = 0; w < kDefThreads / 32; ++w) {
+  for (int w = 0; w < nw; ++w) {
     dmax = fmax(dmax, s_red[0][w]);
     zmax = fmax(zmax, s_red[1][w]);
   }
@@ -344,7 +388,7 @@ __global__ void __launch_bounds__(kDefThreads) merge_deflate_kernel(LevelArgs a)
   int* d_ = a.desc + 8 * m;
   if (rho * zmax <= tol) {
     // everything deflates: the merged order is the result
-    for (int k = tid; k < N; k += kDefThreads) {
+    for (int k = tid; k < N; k += nthr) {
       a.dD[lo + k] = ds[k];
       a.colD[lo + k] = perm[k];
     }
@@ -358,104 +402,176 @@ __global__ void __launch_bounds__(kDefThreads) merge_deflate_kernel(LevelArgs a)
     }
     return;
   }
-  // scan state (thread 0 only)
-  int K = 0, nd = 0, nr = 0, c1 = 0, c2 = 0, c3 = 0;
-  bool have = false;
-  double pd = 0.0, pz = 0.0;
-  int pc = 0, pt = 0;
-  auto emit_root = [&](double dv, double zv, int cv, int tv) {
-    a.dK[lo + K] = dv;
-    a.zK[lo + K] = zv;
-    a.colK[lo + K] = cv;
-    a.typK[lo + K] = tv;
-    a.pT[lo + K] = (tv == 1) ? c1++ : ((tv == 2) ? c2++ : c3++);  // index within its type
-    ++K;
+  // the rotation that merges the survivor (pd, pz) into (dk, zk), if the pair
+  // is close enough
+  auto close_pair = [&](double pd, double pz, double dk, double zk, double& cv, double& sv,
+                        double& tau) {
+    tau = hypot(zk, pz);
+    cv = zk / tau;
+    sv = -pz / tau;
+    return fabs((dk - pd) * cv * sv) <= tol;
   };
-  for (int c0 = 0; c0 < N; c0 += kDefChunk) {
-    const int cn = min(kDefChunk, N - c0);
-    __syncthreads();  // previous chunk consumed
-    for (int k = tid; k < cn; k += kDefThreads) {
-      s_d[k] = ds[c0 + k];
-      s_z[k] = zs[c0 + k];
-      s_c[k] = perm[c0 + k];
-    }
-    __syncthreads();
-    if (tid == 0 && !s_bad) {
-      for (int k = 0; k < cn; ++k) {
-        const double dk = s_d[k], zk = s_z[k];
-        const int ck = s_c[k];
-        if (ck < 0 || ck >= N) {
-          atomicCAS(a.err, 0, kDevBadShape);
-          s_bad = 1;
-          break;
-        }
-        const int tk = (ck < n1) ? 1 : 3;
-        if (rho * fabs(zk) <= tol) {
-          a.dD[lo + nd] = dk;
-          a.colD[lo + nd] = ck;
-          ++nd;
-          continue;
-        }
-        if (!have) {
-          have = true;
-          pd = dk; pz = zk; pc = ck; pt = tk;
-          continue;
-        }
-        double sv = pz, cv = zk;
-        const double tau = hypot(cv, sv);
-        const double t = dk - pd;
-        cv /= tau;
-        sv = -sv / tau;
-        if (fabs(t * cv * sv) <= tol) {
-          // rotate columns (pc, ck): x' = c x + s y, y' = c y - s x
-          a.rA[lo + nr] = pc;
-          a.rB[lo + nr] = ck;
-          a.rc[lo + nr] = cv;
-          a.rs[lo + nr] = sv;
-          ++nr;
-          const double cc = cv * cv, ss = sv * sv;
-          const double dnew_p = pd * cc + dk * ss;
-          const double dnew_k = pd * ss + dk * cc;
-          const int tnew = (pt == tk) ? tk : 2;
-          a.dD[lo + nd] = dnew_p;  // the previous entry deflates
-          a.colD[lo + nd] = pc;
-          ++nd;
-          pd = dnew_k; pz = tau; pc = ck; pt = tnew;
-        } else {
-          emit_root(pd, pz, pc, pt);
-          pd = dk; pz = zk; pc = ck; pt = tk;
-        }
+  int K = 0, nd = 0, c1 = 0, c2 = 0, c3 = 0;  // the same in every thread
+  bool have = false;                          // entry 0 holds a survivor
+  // entry e leaves the scan as a root
+  auto emit_root = [&](int at, int e, int tv, int idx) {
+    a.dK[lo + at] = s_d[e];
+    a.zK[lo + at] = s_z[e];
+    a.colK[lo + at] = s_c[e];
+    a.typK[lo + at] = tv;
+    a.pT[lo + at] = idx;  // index within its type
+  };
+  for (int c0 = 0; c0 < N; c0 += nthr) {
+    const int k = c0 + tid, e = tid + 1;
+    const bool in = k < N;
+    double dk = 0.0, zk = 0.0;
+    int ck = 0;
+    if (in) {
+      dk = ds[k];
+      zk = zs[k];
+      ck = perm[k];
+      if (ck < 0 || ck >= N) {
+        atomicCAS(a.err, 0, kDevBadShape);
+        s_bad = 1;
+        ck = 0;
       }
     }
+    s_d[e] = dk;
+    s_z[e] = zk;
+    s_c[e] = ck;
+    s_t[e] = (ck < n1) ? 1 : 3;
+    s_rot[e] = 0;
+    const bool live = in && !(rho * fabs(zk) <= tol);
+    const unsigned lb = __ballot_sync(0xffffffffu, live);
+    if (lane == 0) s_live[wid] = lb;
+    __syncthreads();
+    if (s_bad) return;
+    // the neighbouring live entries of the chunk (0: the pending one; -1: none)
+    int prev = have ? 0 : -1, next = -1;
+    {
+      unsigned b = lb & ((1u << lane) - 1u);
+      for (int w = wid; w >= 0; --w, b = (w >= 0) ? s_live[w] : 0u)
+        if (b) {
+          prev = 32 * w + 32 - __clz(b);
+          break;
+        }
+      b = lb & ~((2u << lane) - 1u);
+      for (int w = wid; w < nw; ++w, b = (w < nw) ? s_live[w] : 0u)
+        if (b) {
+          next = 32 * w + __ffs(b);
+          break;
+        }
+    }
+    s_prev[e] = prev;
+    s_next[e] = next;
+    double cv, sv, tau;
+    const bool cand = live && prev >= 0 && close_pair(s_d[prev], s_z[prev], dk, zk, cv, sv, tau);
+    const unsigned cb = __ballot_sync(0xffffffffu, cand);
+    if (lane == 0) s_cand[wid] = cb;
+    if (__syncthreads_or(cand) && tid == 0) {
+      int nr = s_nr;
+      for (int w = 0; w < nw; ++w)
+        while (s_cand[w]) {
+          int q = 32 * w + __ffs(s_cand[w]);  // the next entry that rotates
+          int p = s_prev[q];
+          while (close_pair(s_d[p], s_z[p], s_d[q], s_z[q], cv, sv, tau)) {
+            // rotate columns (p, q): x' = c x + s y, y' = c y - s x
+            a.rA[lo + nr] = s_c[p];
+            a.rB[lo + nr] = s_c[q];
+            a.rc[lo + nr] = cv;
+            a.rs[lo + nr] = sv;
+            ++nr;
+            const double cc = cv * cv, ss = sv * sv, pd = s_d[p], qd = s_d[q];
+            s_dp[q] = pd * cc + qd * ss;  // the previous entry deflates
+            s_d[q] = pd * ss + qd * cc;
+            s_z[q] = tau;
+            if (s_t[p] != s_t[q]) s_t[q] = 2;
+            s_rot[q] = 1;
+            s_cand[(q - 1) >> 5] &= ~(1u << ((q - 1) & 31));
+            p = q;
+            q = s_next[q];
+            if (q < 0) break;
+          }
+          // the entry after the run was tested against its changed neighbour
+          if (q >= 0) s_cand[(q - 1) >> 5] &= ~(1u << ((q - 1) & 31));
+        }
+      s_nr = nr;
+    }
+    __syncthreads();
+    const bool rot = live && s_rot[e];
+    int total;
+    // deflated at this entry: itself (small z) or its predecessor (rotation)
+    const bool defl = in && (!live || rot);
+    const int id = nd + block_prefix(defl, s_cnt, &total);
+    nd += total;
+    if (defl) {
+      a.dD[lo + id] = live ? s_dp[e] : dk;
+      a.colD[lo + id] = live ? s_c[prev] : ck;
+    }
+    // its predecessor becomes a root
+    const bool root = live && prev >= 0 && !rot;
+    const int tp = root ? s_t[prev] : 0;
+    const int ir = K + block_prefix(root, s_cnt, &total);
+    K += total;
+    int idx = 0, i1 = block_prefix(tp == 1, s_cnt, &total);
+    if (tp == 1) idx = c1 + i1;
+    c1 += total;
+    i1 = block_prefix(tp == 2, s_cnt, &total);
+    if (tp == 2) idx = c2 + i1;
+    c2 += total;
+    i1 = block_prefix(tp == 3, s_cnt, &total);
+    if (tp == 3) idx = c3 + i1;
+    c3 += total;
+    if (root) emit_root(ir, prev, tp, idx);
+    // the chunk's last live entry is pending
+    int tail = -1;
+    for (int w = nw - 1; w >= 0; --w)
+      if (s_live[w]) {
+        tail = 32 * w + 32 - __clz(s_live[w]);
+        break;
+      }
+    __syncthreads();
+    if (tail > 0) {
+      have = true;
+      if (tid == 0) {
+        s_d[0] = s_d[tail];
+        s_z[0] = s_z[tail];
+        s_c[0] = s_c[tail];
+        s_t[0] = s_t[tail];
+      }
+    }
+    __syncthreads();
+  }
+  if (have) {
+    const int tv = s_t[0];
+    if (tid == 0) emit_root(K, 0, tv, (tv == 1) ? c1 : (tv == 2) ? c2 : c3);
+    c1 += tv == 1;
+    c2 += tv == 2;
+    c3 += tv == 3;
+    ++K;
   }
   if (tid == 0) {
-    if (have && !s_bad) emit_root(pd, pz, pc, pt);
-    s_K = K;
-    s_K1 = c1;
-    s_K2 = c2;
     d_[D_K] = K;
     d_[D_K1] = c1;
     d_[D_K2] = c2;
     d_[D_K3] = c3;
     d_[D_NDEF] = nd;
-    d_[D_NROT] = nr;
+    d_[D_NROT] = s_nr;
   }
   __syncthreads();
-  if (s_bad) return;
   // type-ordered positions for the two structured GEMMs:
   // type 1 -> Qt column c1; type 2 -> Qt column K1 + c2 and Qb column c2;
   // type 3 -> Qb column K2 + c3
-  const int Kf = s_K, K1f = s_K1, K2f = s_K2;
-  for (int i = tid; i < Kf; i += kDefThreads) {
+  for (int i = tid; i < K; i += nthr) {
     const int tv = a.typK[lo + i], idx = a.pT[lo + i];
     if (tv == 1) {
       a.pB[lo + i] = -1;
     } else if (tv == 2) {
-      a.pT[lo + i] = K1f + idx;
+      a.pT[lo + i] = c1 + idx;
       a.pB[lo + i] = idx;
     } else {
       a.pT[lo + i] = -1;
-      a.pB[lo + i] = K2f + idx;
+      a.pB[lo + i] = c2 + idx;
     }
   }
 }
@@ -483,14 +599,21 @@ __global__ void merge_rotate_kernel(LevelArgs a) {
 
 // Gather Q1/mixed columns (top rows) and mixed/Q2 columns (bottom rows) into
 // zero-padded Qt (n1 x K12max) and Qb (n2 x K23max).  grid (ceil(N/256),
-// ceil(Kcols/kColChunk), nm): thread = row, blockIdx.y = a chunk of columns.
-constexpr int kColChunk = 64;
+// ceil(Kcols/chunk), nm): thread = row, blockIdx.y = a chunk of columns.
+// The columns of a chunk are copied one after the other: 64 of them when that
+// still gives every SM a few CTAs, else down to 8 (n = 1000: 20 -> 8 us each).
+int col_chunk(int N, int cols, int nm) {
+  int c = 64;
+  while (c > 8 && (long)ceil_div_i(N, 256) * ceil_div_i(cols, c) * nm < 4L * device_sm_count())
+    c /= 2;
+  return c;
+}
 
 __global__ void merge_gather_kernel(LevelArgs a) {
   const int m = blockIdx.z;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= a.N) return;
-  const int j0 = blockIdx.y * kColChunk;
+  const int j0 = blockIdx.y * a.chunk;
   const long lo = (long)m * a.N;
   const int* d_ = a.desc + 8 * m;
   const int K = d_[D_K], K1 = d_[D_K1], K2 = d_[D_K2], K3 = d_[D_K3];
@@ -498,13 +621,13 @@ __global__ void merge_gather_kernel(LevelArgs a) {
   double* Qt = a.Qt + (long)m * a.n1 * a.K12max;
   double* Qb = a.Qb + (long)m * a.n2 * a.K23max;
   if (r < a.n1) {
-    for (int j = max(j0, K1 + K2); j < min(a.K12max, j0 + kColChunk); ++j)
+    for (int j = max(j0, K1 + K2); j < min(a.K12max, j0 + a.chunk); ++j)
       Qt[r + (long)j * a.n1] = 0.0;
   } else {
-    for (int j = max(j0, K2 + K3); j < min(a.K23max, j0 + kColChunk); ++j)
+    for (int j = max(j0, K2 + K3); j < min(a.K23max, j0 + a.chunk); ++j)
       Qb[(r - a.n1) + (long)j * a.n2] = 0.0;
   }
-  const int i1 = min(K, j0 + kColChunk);
+  const int i1 = min(K, j0 + a.chunk);
   for (int i = j0; i < i1; ++i) {
     long col = a.colK[lo + i];
     if (col < 0 || col >= a.N) {
@@ -524,12 +647,12 @@ __global__ void merge_gather_kernel(LevelArgs a) {
 
 // Deflated columns (after the rotations) -> Zn[:, K + t].  Runs after the
 // merge GEMMs, which write Zn[:, 0:Kmax] for every merge of the level.
-// grid (ceil(N/256), ceil(N/kColChunk), nm).
+// grid (ceil(N/256), ceil(N/chunk), nm).
 __global__ void merge_copy_deflated_kernel(LevelArgs a) {
   const int m = blockIdx.z;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= a.N) return;
-  const int t0 = blockIdx.y * kColChunk;
+  const int t0 = blockIdx.y * a.chunk;
   const long lo = (long)m * a.N;
   const int* d_ = a.desc + 8 * m;
   const int K = d_[D_K], nd = d_[D_NDEF];
@@ -539,7 +662,7 @@ __global__ void merge_copy_deflated_kernel(LevelArgs a) {
     atomicCAS(a.err, 0, kDevBadShape);
     return;
   }
-  const int t1 = min(nd, t0 + kColChunk);
+  const int t1 = min(nd, t0 + a.chunk);
   for (int t = t0; t < t1; ++t) {
     long col = a.colD[lo + t];
     if (col < 0 || col >= a.N) {
@@ -790,12 +913,12 @@ __global__ void merge_finalize_rank_kernel(LevelArgs a) {
 }
 
 // Zw[lo:hi, lo + p] = Zn[:, perm[p]], dw[lo + p] = sorted value.
-// grid (ceil(N/256), ceil(N/kColChunk), nm): thread = row, blockIdx.y = columns.
+// grid (ceil(N/256), ceil(N/chunk), nm): thread = row, blockIdx.y = columns.
 __global__ void merge_scatter_kernel(LevelArgs a) {
   const int m = blockIdx.z;
-  const int p0 = blockIdx.y * kColChunk;
+  const int p0 = blockIdx.y * a.chunk;
   const long lo = (long)m * a.N;
-  const int p1 = min(a.N, p0 + kColChunk);
+  const int p1 = min(a.N, p0 + a.chunk);
   if (blockIdx.x == 0 && p0 + (int)threadIdx.x < p1)
     a.dw[lo + p0 + threadIdx.x] = a.zv[lo + p0 + threadIdx.x];
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -880,8 +1003,8 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
   EVD_LAUNCHED();
   EVD_CUDA_TRY(cudaMemsetAsync(Zw, 0, sizeof(double) * np * np, st));
   const int nleaves = 1 << P.L;
-  leaf_ql_kernel<<<ceil_div_i((long)nleaves * 32, 128), 128, 0, st>>>(P.s, nleaves, dw, ew, Zw,
-                                                                       np, err);
+  leaf_ql_kernel<<<ceil_div_i(nleaves, kLeafWarps), 32 * kLeafWarps, 0, st>>>(
+      P.s, nleaves, dw, ew, Zw, np, err);
   EVD_LAUNCHED();
 
   std::vector<int> hdesc;
@@ -926,7 +1049,7 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
     dim3 gN(ceil_div_i(a.N, 256), a.nm);
     merge_setup_kernel<<<gN, 256, 0, st>>>(a);
     EVD_LAUNCHED();
-    merge_deflate_kernel<<<a.nm, kDefThreads, 0, st>>>(a);
+    merge_deflate_kernel<<<a.nm, std::min(kDefMax, (a.N + 31) / 32 * 32), 0, st>>>(a);
     EVD_LAUNCHED();
     hdesc.resize(8 * a.nm);
     EVD_CUDA_TRY(cudaMemcpyAsync(hdesc.data(), a.desc, sizeof(int) * 8 * a.nm,
@@ -953,7 +1076,8 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
     {
       const int cols = std::max(Kmax, std::max(a.K12max, a.K23max));
       if (cols > 0) {
-        dim3 gG(ceil_div_i(a.N, 256), ceil_div_i(cols, kColChunk), a.nm);
+        a.chunk = col_chunk(a.N, cols, a.nm);
+        dim3 gG(ceil_div_i(a.N, 256), ceil_div_i(cols, a.chunk), a.nm);
         merge_gather_kernel<<<gG, 256, 0, st>>>(a);
         EVD_LAUNCHED();
       }
@@ -1005,7 +1129,8 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
         }
       }
     }
-    dim3 gC(ceil_div_i(a.N, 256), ceil_div_i(a.N, kColChunk), a.nm);
+    a.chunk = col_chunk(a.N, a.N, a.nm);
+    dim3 gC(ceil_div_i(a.N, 256), ceil_div_i(a.N, a.chunk), a.nm);
     merge_copy_deflated_kernel<<<gC, 256, 0, st>>>(a);
     EVD_LAUNCHED();
     merge_finalize_rank_kernel<<<gN, 256, 0, st>>>(a);

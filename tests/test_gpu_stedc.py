@@ -86,3 +86,19 @@ def test_stedc_scaling(cuda, evdlib):
     rng = np.random.default_rng(11)
     for s in (1e-150, 1e150):
         _check(cuda, evdlib, s * rng.standard_normal(300), s * rng.standard_normal(299))
+
+
+@pytest.mark.parametrize("n", [1023, 1025, 2500, 4100])
+@pytest.mark.parametrize("kind", ["wilkinson", "clusters", "mixed"])
+def test_stedc_rotation_runs(cuda, evdlib, n, kind):
+    """Merges longer than one deflation chunk (1024 entries) with runs of close
+    pairs, many of them across the chunk boundaries."""
+    rng = np.random.default_rng(n)
+    if kind == "wilkinson":  # close pairs everywhere
+        d, e = np.abs(np.arange(n) - n // 2).astype(float), np.ones(n - 1)
+    elif kind == "clusters":  # long runs of equal eigenvalues, weakly coupled
+        d, e = np.repeat(np.arange(n // 50 + 1.0), 50)[:n], np.full(n - 1, 1e-9)
+    else:  # equal blocks between random ones
+        d, e = rng.standard_normal(n), rng.standard_normal(n - 1)
+        d[n // 3: 2 * n // 3], e[n // 3: 2 * n // 3] = 0.25, 1e-17
+    _check(cuda, evdlib, d, e)
