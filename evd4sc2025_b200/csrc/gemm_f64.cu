@@ -701,13 +701,16 @@ static int gemm_run(GemmArgs p, bool ta, bool tb, long batch, cudaStream_t st,
 
 int choose_splitk(long m, long n, long k, long batch) {
   // Enough CTAs for about four per SM when the output is small and K long
-  // (eight for the n <= 32 panel products, measured best on B200).
+  // (eight for the n <= 32 panel products, measured best on B200).  A split
+  // keeps at least 64 of K (four k-tiles): these products are bound by the
+  // latency of their k-tile chain, so with 256 a 1024 x 32 x 1024 product ran
+  // on 48 CTAs and took 12 us.
   const long bm = 64, bn = (n <= 32) ? 32 : 64;
   long tiles = ((m + bm - 1) / bm) * ((n + bn - 1) / bn) * batch;
   long want = ((n <= 32) ? 8L : 4L) * device_sm_count();
-  if (tiles >= want || k < 512) return 1;
+  if (tiles >= want || k < 128) return 1;
   long s = (want + tiles - 1) / tiles;
-  long kmax = k / 256;  // keep >= 256 of K per split
+  const long kmax = (n <= 32) ? std::min(k / 64, std::max(k / 256, 512 / tiles)) : k / 256;
   if (s > kmax) s = kmax;
   if (s > 32) s = 32;
   return (int)std::max<long>(1, s);

@@ -76,7 +76,8 @@ static Sy2sbLayout sy2sb_layout(long M, long b, long nb) {
   L.s2_off = L.s1_off + L.small_n;
   L.s3_off = L.s2_off + L.small_n;
   L.sk_off = L.s3_off + L.small_n;
-  L.sk_n = std::max(8 * M * b, 32 * nb * b);
+  // partial sums: up to 32 splits of the small products, 8 of the largest
+  L.sk_n = std::max({8 * M * b, 32 * nb * b, 32 * std::min(M, 2048L) * b});
   L.total = L.sk_off + L.sk_n;
   return L;
 }
