@@ -88,3 +88,22 @@ def test_values_only_any_order(cuda, evdlib, n, nb):
     assert w.shape == (n,)
     ref = np.linalg.eigvalsh(A)
     assert np.abs(w.cpu().numpy() - ref).max() <= 1e-12 * max(np.linalg.norm(A, 2), 1e-300)
+
+
+@pytest.mark.parametrize("n", [7, 8, 9, 16, 65])
+@pytest.mark.parametrize("kind", ["constant", "decoupled", "tiny", "zero_diagonal"])
+def test_stebz_vanishing_terms(cuda, evdlib, kind, n):
+    """Rows where a term of the Sturm sequence vanishes or underflows."""
+    rng = np.random.default_rng(n)
+    d, e = rng.standard_normal(n), rng.standard_normal(n - 1)
+    if kind == "constant":
+        d, e = np.full(n, 0.5), np.zeros(n - 1)
+    elif kind == "decoupled":
+        d, e = np.round(2 * d) / 2, np.where(np.arange(n - 1) % 3 == 0, 0.0, np.round(2 * e) / 2)
+    elif kind == "tiny":
+        d, e = np.where(np.arange(n) % 4 == 0, d, 1e-180 * d), 1e-170 * e
+    else:
+        d = np.zeros(n)
+    w = evdlib.stebz(torch.from_numpy(d).to(cuda), torch.from_numpy(e).to(cuda)).cpu().numpy()
+    w_ref = O.tridiag_eig(d, e)[0]
+    assert np.abs(w - w_ref).max() <= 1e-13 * max(np.abs(w_ref).max(), 1e-300) * np.sqrt(n)
