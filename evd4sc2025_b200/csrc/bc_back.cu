@@ -46,6 +46,8 @@
 
 namespace evd {
 
+int* pool_ints(long count, cudaStream_t st);
+
 namespace {
 
 constexpr int kQW = 4;                   // warps per CTA
@@ -510,9 +512,10 @@ __global__ void __launch_bounds__(kQThreads, 2)
 // {1, 3, 5, 7} (x[i][1]) with the B operand read from the same staged
 // reflector segments; W (column g, reflectors 2t, 2t+1) is in turn the A
 // operand of the update for the even and odd reflectors against the -V
-// fragments.  The window takes 68 registers instead of 136, so twice as many
-// warps share each sub-partition's tensor pipe (the kernel above is bound by
-// its dependent DMMA chains with two warps per sub-partition).
+// fragments.  The window takes 68 registers instead of 136 and the staging ring
+// two buffers instead of three (a block lasts far longer than the copies), so
+// three warps instead of two share each sub-partition's tensor pipe (the kernel
+// above is bound by its dependent DMMA chains with two).
 constexpr int kQ8Cols = 8;
 
 __device__ __forceinline__ void w_part8(const double (&x)[kTiles][2], const double* ys, int offW,
@@ -565,11 +568,12 @@ __device__ __forceinline__ void apply_block8(double (&x)[kTiles][2], const doubl
   }
 }
 
+template <bool L2>
 __device__ __forceinline__ void load_tile8(double (&v)[2], const double* cg, bool ok, long row0,
                                            int t2, int n) {
   const long r = row0 + t2;
-  v[0] = (ok && r >= 0 && r < n) ? cg[r] : 0.0;
-  v[1] = (ok && r + 1 >= 0 && r + 1 < n) ? cg[r + 1] : 0.0;
+  v[0] = (ok && r >= 0 && r < n) ? (L2 ? __ldcg(cg + r) : cg[r]) : 0.0;
+  v[1] = (ok && r + 1 >= 0 && r + 1 < n) ? (L2 ? __ldcg(cg + r + 1) : cg[r + 1]) : 0.0;
 }
 __device__ __forceinline__ void store_tile8(const double (&v)[2], double* cg, bool ok, long row0,
                                             int t2, int n) {
@@ -578,19 +582,60 @@ __device__ __forceinline__ void store_tile8(const double (&v)[2], double* cg, bo
   if (ok && r + 1 >= 0 && r + 1 < n) cg[r + 1] = v[1];
 }
 
-template <bool FWD, int NW, bool RANGE>
-__global__ void __launch_bounds__(NW * 32, 2)
+// PIPE: one CTA per (strip, column block) instead of one per column block.  A
+// strip needs of the strip processed before it only rows that are final there
+// a few blocks earlier: block `it` of a strip slides in a tile that the other
+// strip has stored after it + 2 (forward) or it + 18 (reverse) of its blocks,
+// so the strips of a column block run concurrently, one behind the other.
+// CTAs take their work from a ticket, strip by strip, and wait only for a
+// strip that an earlier ticket owns, so some CTA can always go on.  prog[] holds
+// the blocks that each (strip, column block) has finished (its count + 1 at the
+// end), ticket and counters start at zero.  A wait that outlasts 4 s fills the
+// columns with NaN (nothing else could report it from here).
+// X passes between SMs, so PIPE reads it past L1.
+struct Q2Pipe {
+  int* ticket;
+  int* prog;
+};
+constexpr int kPubEvery = 4;  // blocks between two publications of progress
+
+__device__ __forceinline__ bool q2_wait(const int* flag, int need, int& seen) {
+  if (seen >= need) return true;
+  unsigned long long t0 = 0;
+  for (unsigned it = 1;; ++it) {
+    seen = ld_acquire(flag);
+    if (seen >= need) return true;
+    if ((it & 1023u) == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (t0 == 0) t0 = t;
+      if (t - t0 > 4000000000ull) return false;
+    }
+  }
+}
+
+template <bool FWD, int NW, bool RANGE, bool PIPE>
+__global__ void __launch_bounds__(NW * 32, 3)
     q2_mma8_kernel(int n, int ncols, const double* __restrict__ U, long ldU,
-                   const double* __restrict__ Tg, double* __restrict__ X, long ldX, Q2Range rg) {
+                   const double* __restrict__ Tg, double* X, long ldX, Q2Range rg, Q2Pipe pp) {
   extern __shared__ __align__(16) double smem[];
-  double* Ys = smem;                 // kNYBuf x kYBuf
-  double* Ts = Ys + kNYBuf * kYBuf;  // kNYBuf x kVBuf (-V fragments)
+  double* Ys = smem;            // 2 x kYBuf
+  double* Ts = Ys + 2 * kYBuf;  // 2 x kVBuf (-V fragments)
   const int nthr = NW * 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  for (int e = threadIdx.x; e < kNYBuf * kYBuf; e += nthr) Ys[e] = 0.0;
+  for (int e = threadIdx.x; e < 2 * kYBuf; e += nthr) Ys[e] = 0.0;
   const int offW = seg_off(g, 0) + 2 * t - g;  // Y[8i+2t(+1)][g]
-  const int cblk = (RANGE && rg.rev) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+  const int ncb = (ncols + NW * kQ8Cols - 1) / (NW * kQ8Cols);  // column blocks
+  int item = 0;
+  if (PIPE) {
+    __shared__ int s_item;
+    if (threadIdx.x == 0) s_item = atomicAdd(pp.ticket, 1);
+    __syncthreads();
+    item = s_item;
+  }
+  const int cb_at = PIPE ? item % ncb : (int)blockIdx.x;
+  const int cblk = (RANGE && rg.rev) ? ncb - 1 - cb_at : cb_at;
   const int c0 = cblk * (NW * kQ8Cols) + warp * kQ8Cols;
   const bool okg = c0 + g < ncols;
   double* cg = X + (long)(okg ? c0 + g : 0) * ldX;
@@ -615,7 +660,9 @@ __global__ void __launch_bounds__(NW * 32, 2)
   };
   const long cta_col0 = (long)cblk * (NW * kQ8Cols);
   const int ns = RANGE ? q2_strips(rg, n, nstrips, cta_col0, NW * kQ8Cols) : nstrips;
-  for (int si = 0; si < ns; ++si) {
+  const int s_beg = PIPE ? item / ncb : 0;
+  const int s_end = PIPE ? min(ns, s_beg + 1) : ns;
+  for (int si = s_beg; si < s_end; ++si) {
     const int sidx = FWD ? (ns - 1 - si) : si;
     const long R = (long)sidx * kStrip;
     const int H = n - 2 - (int)R;
@@ -623,38 +670,62 @@ __global__ void __launch_bounds__(NW * 32, 2)
     const int bbA = RANGE ? rg.h0 / 8 : 0, bbB = RANGE ? min(nblk, (rg.h1 + 7) / 8) : nblk;
     const int cnt = bbB - bbA;
     auto bb_of = [&](int it) { return FWD ? (bbA + it) : (bbB - 1 - it); };
+    // the strip processed before this one, and its number of blocks
+    const bool dep = PIPE && si > 0;
+    const int* dflag = dep ? pp.prog + (long)(si - 1) * ncb + cb_at : nullptr;
+    int* mine = PIPE ? pp.prog + (long)si * ncb + cb_at : nullptr;
+    int cnt_d = 0, seen = 0;
+    bool ok = true;
+    if (dep) {
+      const int nb_d = nblk + (FWD ? -kStrip / 8 : kStrip / 8);
+      cnt_d = (RANGE ? min(nb_d, (rg.h1 + 7) / 8) : nb_d) - bbA;
+    }
+    // blocks of it that have to be finished before iteration `it` slides in its
+    // tile (-1: the first window); the tile that only the final frame holds
+    // needs the whole strip
+    auto need_of = [&](int it) {
+      const int k = FWD ? it + 2 : it + 18;
+      return (it >= cnt - 1 || k > cnt_d) ? cnt_d + 1 : k;
+    };
 
-    __syncthreads();
+    if (PIPE && dep && threadIdx.x == 0) ok = q2_wait(dflag, need_of(-1), seen);
+    if (PIPE) {
+      ok = __syncthreads_and(ok) != 0;
+      if (!ok) {
+        for (int i = 0; i < n; ++i)
+          if (okg && t == 0) cg[i] = __longlong_as_double(0x7ff8000000000000ll);
+        __syncthreads();
+        if (threadIdx.x == 0) st_release(mine, cnt + 1);
+        return;
+      }
+    } else {
+      __syncthreads();
+    }
     {
       const long base = R + 8L * bb_of(0) + 1;
 #pragma unroll
-      for (int i = 0; i < kTiles; ++i) load_tile8(x[i], cg, okg, base + 8 * i, t2, n);
+      for (int i = 0; i < kTiles; ++i) load_tile8<PIPE>(x[i], cg, okg, base + 8 * i, t2, n);
     }
     stage_y(Ys, R, H, bb_of(0));
     stage_t(Ts, sidx, bb_of(0));
     cp_commit();
-    if (cnt > 1) {
-      stage_y(Ys + kYBuf, R, H, bb_of(1));
-      stage_t(Ts + kVBuf, sidx, bb_of(1));
-    }
-    cp_commit();
-    cp_wait<1>();
-    __syncthreads();
 
 #pragma unroll 1
     for (int it = 0; it < cnt; ++it) {
       const int bb = bb_of(it);
       const long base = R + 8L * bb + 1;
       cp_wait<0>();
+      if (PIPE && dep && ok && threadIdx.x == 0) ok = q2_wait(dflag, need_of(it), seen);
       __syncthreads();
-      if (it + 2 < cnt) {
-        stage_y(Ys + ((it + 2) % 3) * kYBuf, R, H, bb_of(it + 2));
-        stage_t(Ts + ((it + 2) % 3) * kVBuf, sidx, bb_of(it + 2));
+      if (PIPE && threadIdx.x == 0 && it > 0 && it % kPubEvery == 0) st_release(mine, it);
+      if (it + 1 < cnt) {
+        stage_y(Ys + ((it + 1) & 1) * kYBuf, R, H, bb_of(it + 1));
+        stage_t(Ts + ((it + 1) & 1) * kVBuf, sidx, bb_of(it + 1));
       }
       cp_commit();
       double inc[2];
-      load_tile8(inc, cg, okg, FWD ? (base + 8 * kTiles) : (base - 8), t2, n);
-      apply_block8<FWD>(x, Ys + (it % 3) * kYBuf, Ts + (it % 3) * kVBuf, lane, offW);
+      load_tile8<PIPE>(inc, cg, okg, FWD ? (base + 8 * kTiles) : (base - 8), t2, n);
+      apply_block8<FWD>(x, Ys + (it & 1) * kYBuf, Ts + (it & 1) * kVBuf, lane, offW);
       if (FWD) {
         store_tile8(x[0], cg, okg, base, t2, n);
 #pragma unroll
@@ -680,18 +751,40 @@ __global__ void __launch_bounds__(NW * 32, 2)
 #pragma unroll
       for (int i = 0; i < kTiles; ++i) store_tile8(x[i], cg, okg, base + 8 * i, t2, n);
     }
+    if (PIPE) {
+      if (threadIdx.x == 0 && !ok)  // a wait ran out: visible in the result
+        for (int i = 0; i < n; ++i) cg[i] = __longlong_as_double(0x7ff8000000000000ll);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        __threadfence();
+        st_release(mine, cnt + 1);
+      }
+    }
   }
 }
 
-constexpr size_t kQ8Smem = (size_t)(kNYBuf * kYBuf + kNYBuf * kVBuf) * sizeof(double);
+// Ints of the pipelined kernel's ticket and progress counters.
+long q2_flag_ints(long n, long ncols) {
+  return 4 + ((n - 2 + kStrip - 1) / kStrip) * ((ncols + 31) / 32);
+}
+
+constexpr size_t kQ8Smem = (size_t)2 * (kYBuf + kVBuf) * sizeof(double);  // 4 CTAs fit an SM
 
 template <bool FWD, int NW, bool RANGE>
 int launch_q2_8(long n, long ncols, const double* U, long ldU, const double* Tg, double* X,
-                long ldX, Q2Range rg, cudaStream_t st) {
-  EVD_TRY(smem_attr_once((const void*)q2_mma8_kernel<FWD, NW, RANGE>, (int)kQ8Smem));
-  const int grid = ceil_div_i((int)ncols, NW * kQ8Cols);
-  q2_mma8_kernel<FWD, NW, RANGE><<<grid, NW * 32, kQ8Smem, st>>>((int)n, (int)ncols, U, ldU, Tg,
-                                                                 X, ldX, rg);
+                long ldX, Q2Range rg, int* flags, cudaStream_t st) {
+  const int ncb = ceil_div_i((int)ncols, NW * kQ8Cols);
+  if (flags) {
+    const int nstrips = (int)((n - 2 + kStrip - 1) / kStrip);
+    EVD_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)q2_flag_ints(n, ncols), st));
+    EVD_TRY(smem_attr_once((const void*)q2_mma8_kernel<FWD, NW, RANGE, true>, (int)kQ8Smem));
+    q2_mma8_kernel<FWD, NW, RANGE, true><<<ncb * nstrips, NW * 32, kQ8Smem, st>>>(
+        (int)n, (int)ncols, U, ldU, Tg, X, ldX, rg, Q2Pipe{flags, flags + 4});
+  } else {
+    EVD_TRY(smem_attr_once((const void*)q2_mma8_kernel<FWD, NW, RANGE, false>, (int)kQ8Smem));
+    q2_mma8_kernel<FWD, NW, RANGE, false><<<ncb, NW * 32, kQ8Smem, st>>>(
+        (int)n, (int)ncols, U, ldU, Tg, X, ldX, rg, Q2Pipe{nullptr, nullptr});
+  }
   EVD_LAUNCHED();
   return EVD_SUCCESS;
 }
@@ -707,22 +800,25 @@ int launch_q2(long n, long ncols, const double* U, long ldU, const double* Tg, d
   return EVD_SUCCESS;
 }
 
-// With fewer 64-column CTAs than SMs (ncols < 64 x SMs: n <= 8192 on B200)
-// the 16-column kernel leaves SMs idle; the 8-column kernel (4 warps, 32
-// columns per CTA) doubles the warps (n = 4096: 19.8 -> 14.0 ms).  Above that
-// the 16-column kernel is faster (n = 16384: 436 ms against 461 ms with
-// 8-column warps, whose m8n8k4 operands double the shared-memory reads per
-// flop).  A launch over every sweep without an identity start takes the
-// kernels compiled without the range logic.
+// The 8-column kernel, pipelined over the strips where the caller has the
+// counters for it (three CTAs per SM from the first strip to the last, for any
+// column count): n x ncols, ms, unpipelined -> pipelined: 1000 x 1000 0.93 ->
+// 0.39, 4096 x 4096 14.0 -> 6.8, 6000 x 1500 28.5 -> 5.9, 8192 x 8192 68.7 ->
+// 51.9, 16384 x 16384 461 -> 410 (21.4 TFLOP/s of algorithm, 0.72 of the DMMA
+// rate with the parallelogram padding).  Without counters, the 16-column kernel
+// from 64 columns per SM on (n = 16384: 436 ms), the 8-column one below.  A
+// launch over every sweep without an identity start takes the kernels compiled
+// without the range logic.
 template <bool FWD>
 int launch_q2_pre(long n, long ncols, const double* U, long ldU, const double* Tg, double* X,
-                  long ldX, Q2Range rg, cudaStream_t st) {
+                  long ldX, Q2Range rg, int* flags, cudaStream_t st) {
   const bool whole = !rg.ident && rg.h0 == 0 && rg.h1 >= n - 2;
-  if (ncols >= 64L * device_sm_count())
+  if (n <= kStrip + 2) flags = nullptr;  // a single strip
+  if (!flags && ncols >= 64L * device_sm_count())
     return whole ? launch_q2<FWD, true, false>(n, ncols, U, ldU, Tg, X, ldX, rg, st)
                  : launch_q2<FWD, true, true>(n, ncols, U, ldU, Tg, X, ldX, rg, st);
-  return whole ? launch_q2_8<FWD, 4, false>(n, ncols, U, ldU, Tg, X, ldX, rg, st)
-               : launch_q2_8<FWD, 4, true>(n, ncols, U, ldU, Tg, X, ldX, rg, st);
+  return whole ? launch_q2_8<FWD, 4, false>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, st)
+               : launch_q2_8<FWD, 4, true>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, st);
 }
 
 // -V fragments of the blocks of sweeps [h0, h1) in every strip.
@@ -748,7 +844,8 @@ long q2_tbuf_doubles(long n) {
 }
 
 int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, double* X,
-                   long ldX, double* tbuf, long h0, long h1, long ident_k, cudaStream_t st) {
+                   long ldX, double* tbuf, int* flags, long h0, long h1, long ident_k,
+                   cudaStream_t st) {
   const bool ident = ident_k >= 0;
   if (n < 0 || ncols < 0 || ldU < n || ldX < n) return EVD_ERR_INVALID_ARG;
   if (n > (1L << 30) || ncols > (1L << 30)) return EVD_ERR_INVALID_ARG;
@@ -764,18 +861,24 @@ int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, 
   if (tbuf) {
     if (forward) {
       EVD_TRY(launch_tbuild<true>(n, U, ldU, tbuf, h0, h1, st));
-      return launch_q2_pre<true>(n, ncols, U, ldU, tbuf, X, ldX, rg, st);
+      return launch_q2_pre<true>(n, ncols, U, ldU, tbuf, X, ldX, rg, flags, st);
     }
     EVD_TRY(launch_tbuild<false>(n, U, ldU, tbuf, h0, h1, st));
-    return launch_q2_pre<false>(n, ncols, U, ldU, tbuf, X, ldX, rg, st);
+    return launch_q2_pre<false>(n, ncols, U, ldU, tbuf, X, ldX, rg, flags, st);
   }
   return forward ? launch_q2<true, false, true>(n, ncols, U, ldU, nullptr, X, ldX, rg, st)
                  : launch_q2<false, false, true>(n, ncols, U, ldU, nullptr, X, ldX, rg, st);
 }
 
 int q2_apply(bool forward, long n, long ncols, const double* U, long ldU, double* X, long ldX,
-             double* tbuf, cudaStream_t st) {
-  return q2_apply_range(forward, n, ncols, U, ldU, X, ldX, tbuf, 0, n, -1, st);
+             double* tbuf, int* flags, cudaStream_t st) {
+  return q2_apply_range(forward, n, ncols, U, ldU, X, ldX, tbuf, flags, 0, n, -1, st);
+}
+
+// Ints of the optional `flags` scratch of q2_apply (0: of no use).
+long q2_flags(long n, long ncols) {
+  if (n <= kStrip + 2 || ncols <= 0) return 0;
+  return q2_flag_ints(n, ncols);
 }
 
 }  // namespace evd
@@ -785,12 +888,19 @@ extern "C" long evd_bc_back_work_size(long n) { return evd::q2_tbuf_doubles(n < 
 extern "C" int evd_bc_back(double* Q, long ldQ, const double* U, long ldU, long n, int b,
                            cudaStream_t stream) {
   if (b != 32) return EVD_ERR_INVALID_ARG;
-  return evd::q2_apply(true, n, n, U, ldU, Q, ldQ, nullptr, stream);
+  return evd::q2_apply(true, n, n, U, ldU, Q, ldQ, nullptr, nullptr, stream);
 }
 
 extern "C" int evd_bc_back_apply(long n, long ncols, const double* U, long ldU, double* X,
                                  long ldX, int b, double* work, long lwork, cudaStream_t stream) {
   if (b != 32) return EVD_ERR_INVALID_ARG;
   if (work && lwork < evd::q2_tbuf_doubles(n)) return EVD_ERR_WORKSPACE;
-  return evd::q2_apply(false, n, ncols, U, ldU, X, ldX, work, stream);
+  // the pipelined kernel's counters (a few ints per strip and 32 columns) come
+  // from the library's stream-ordered pool; without them it runs unpipelined
+  int* flags = nullptr;
+  const long nf = work ? evd::q2_flags(n, ncols) : 0;
+  if (nf > 0 && ldU >= n && ldX >= n && U && X) flags = evd::pool_ints(nf, stream);
+  const int rc = evd::q2_apply(false, n, ncols, U, ldU, X, ldX, work, flags, stream);
+  if (flags) EVD_CUDA_TRY(cudaFreeAsync(flags, stream));
+  return rc;
 }

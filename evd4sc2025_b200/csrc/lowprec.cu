@@ -648,6 +648,19 @@ int tc_syr2k_run(long n, long k, float alpha, const TI* A, long lda, const TI* B
 }
 
 }  // namespace
+
+// `count` ints from the pool, freed with cudaFreeAsync; nullptr when there are none.
+int* pool_ints(long count, cudaStream_t st) {
+  cudaMemPool_t pool = lp_pool();
+  int* p = nullptr;
+  if (!pool || cudaMallocFromPoolAsync((void**)&p, sizeof(int) * (size_t)count, pool, st) !=
+                   cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+
 }  // namespace evd
 
 using evd::lp_panel;

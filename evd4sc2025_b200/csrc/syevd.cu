@@ -43,9 +43,11 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
 long stedc_oz_bytes(long n, int nmod);
 long q2_tbuf_doubles(long n);
 int q2_apply(bool forward, long n, long ncols, const double* U, long ldU, double* X, long ldX,
-             double* tbuf, cudaStream_t st);
+             double* tbuf, int* flags, cudaStream_t st);
 int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, double* X,
-                   long ldX, double* tbuf, long h0, long h1, long ident_k, cudaStream_t st);
+                   long ldX, double* tbuf, int* flags, long h0, long h1, long ident_k,
+                   cudaStream_t st);
+long q2_flags(long n, long ncols);
 bool chase_pipelined(long n);
 int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, int* iwork,
                      long s0, long s1, int part, cudaStream_t st);
@@ -252,7 +254,9 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
     // the T factors of the chasing reflectors go into OA (free after stage 1);
     // for very small n they do not fit and the kernel rebuilds them itself
     double* tbuf = ((size_t)q2_tbuf_doubles(n) <= (size_t)n * n) ? OA : nullptr;
-    EVD_TRY(q2_apply(false, n, n, U, n, X, ldX, tbuf, st));
+    // the pipelined kernel's counters into Z (n nb doubles, free after stage 1)
+    int* flags = (q2_flags(n, n) > 0 && q2_flags(n, n) <= 2 * n * nb) ? (int*)Z : nullptr;
+    EVD_TRY(q2_apply(false, n, n, U, n, X, ldX, tbuf, flags, st));
   }
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[4], st));
   {
@@ -429,13 +433,22 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
   // ---- the chains, range by range behind the chase ----
   {
     NvtxRange r("evd_b200 stage-2 reflectors beside the chase (side streams)");
+    // The pipelined kernel's counters into Z and R (free after stage 1).  Where
+    // the 64-column CTAs of the plain kernel fill the SMs it is the better
+    // neighbour of the divide and conquer and the Q1 formation: n = 16384 833 ms
+    // against 859 (three pipelined CTAs per SM leave them no room), 8192 176
+    // against 165.
+    const bool fits = n < 64L * device_sm_count() && q2_flags(n, n) > 0 &&
+                      q2_flags(n, n) <= 2 * n * nb;
+    int* fl[2] = {fits ? (int*)Z : nullptr, fits ? (int*)R : nullptr};
     for (int i = 0; i < nr; ++i) {
       EVD_CUDA_TRY(cudaStreamWaitEvent(sa, evr[i], 0));
-      EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, bounds[i],
-                             split ? k : bounds[i + 1], 0, sa));
+      EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, fl[0],
+                             bounds[i], split ? k : bounds[i + 1], 0, sa));
       if (split) {
         EVD_CUDA_TRY(cudaStreamWaitEvent(sc, evr[i], 0));
-        EVD_TRY(q2_apply_range(true, n, n, U, n, X, ldX, tbuf, k, bounds[i + 1], k, sc));
+        EVD_TRY(q2_apply_range(true, n, n, U, n, X, ldX, tbuf, fl[1], k,
+                               bounds[i + 1], k, sc));
       }
     }
   }

@@ -52,6 +52,28 @@ def test_q2_apply_without_workspace(cuda, evdlib, n, ncols):
     assert np.abs(a - b).max() <= 1e-13 * max(1.0, np.sqrt(n))
 
 
+@pytest.mark.parametrize("n,ncols", [(130, 1), (131, 33), (258, 31), (387, 500), (1100, 32),
+                                     (2100, 700)])
+def test_q2_apply_strips_side_by_side(cuda, evdlib, n, ncols):
+    """The strips of a column block run concurrently: Q2^T (Q2 X) = X for both
+    directions (the workspace path), and the result of the path without
+    workspace, which takes the strips one after the other."""
+    g = torch.Generator(device=cuda).manual_seed(n)
+    sub = torch.zeros(n, 64, dtype=torch.float64, device=cuda)
+    for o in range(33):
+        sub[: n - o, o] = torch.randn(n - o, generator=g, dtype=torch.float64, device=cuda)
+    _, _, U = evdlib.bulge_chase(sub.t(), 32)
+    X = evdlib.to_cm(torch.randn(n, ncols, generator=g, dtype=torch.float64, device=cuda),
+                     device=cuda)
+    a, b = X.clone(memory_format=torch.preserve_format), X.clone(
+        memory_format=torch.preserve_format)
+    evdlib.bc_back_apply(a, U, work=True)
+    evdlib.bc_back_apply(b, U, work=None)
+    assert (a - b).abs().max() <= 1e-13 * np.sqrt(n) * X.abs().max()
+    _fwd(evdlib, a, U)
+    assert (a - X).abs().max() <= 1e-12 * np.sqrt(n)
+
+
 def test_q2_apply_rejects_small_workspace(cuda, evdlib):
     import ctypes as C
     n = 300
