@@ -86,26 +86,46 @@ __global__ void lambda_kernel(long n, const double* __restrict__ S, long lds, do
   if ((threadIdx.x & 31) == 0) atomic_max_nonneg(scal, m);
 }
 
-// y = M v for M = S - diag(lam) (which = 0) or M = R (which = 1); one warp per
-// column j (M symmetric: y_j = column j . v), coalesced column reads.
-__global__ void symv_kernel(long n, const double* __restrict__ M, long ldm,
-                            const double* __restrict__ lam, const double* __restrict__ v,
-                            double* __restrict__ y, int sub_diag) {
+// One power-iteration product of both matrices: y0 = (S - diag(lam)) v0 and
+// y1 = R v1 (gridDim.y = 2), one warp per column (both symmetric: y_j = column
+// j . v).  Bound by reading S and R; eight loads per lane in flight and both
+// matrices in one launch (n = 3072: 24 us against 2 x 47 us with one load per
+// lane at a time).
+__global__ void __launch_bounds__(256)
+    symv_kernel(long n, const double* __restrict__ S, const double* __restrict__ R, long ldm,
+                const double* __restrict__ lam, const double* __restrict__ v0,
+                const double* __restrict__ v1, double* __restrict__ y0, double* __restrict__ y1) {
+  const bool first = blockIdx.y == 0;
+  const double* M = first ? S : R;
+  const double* v = first ? v0 : v1;
+  double* y = first ? y0 : y1;
   const long warps = (long)gridDim.x * (blockDim.x >> 5);
   const int lane = threadIdx.x & 31;
   for (long j = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5); j < n; j += warps) {
     const double* col = M + j * ldm;
-    double acc = 0.0;
-    for (long i = lane; i < n; i += 32) acc = fma(col[i], v[i], acc);
-    acc = warp_sum(acc);
-    if (lane == 0) y[j] = sub_diag ? acc - lam[j] * v[j] : acc;
+    double acc[8] = {};
+    long i = lane;
+    for (; i + 7 * 32 < n; i += 8 * 32) {
+      double c[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) c[q] = __ldcs(col + i + 32 * q);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] = fma(c[q], __ldg(v + i + 32 * q), acc[q]);
+    }
+    for (; i < n; i += 32) acc[0] = fma(col[i], v[i], acc[0]);
+    double t = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+    t = warp_sum(t);
+    if (lane == 0) y[j] = first ? t - lam[j] * v[j] : t;
   }
 }
 
-// v = y / ||y||; out = ||y|| (single block)
-__global__ void normalize_kernel(long n, const double* __restrict__ y, double* __restrict__ v,
-                                 double* out) {
+// v = y / ||y||; out = ||y||, for both vectors (one block each)
+__global__ void normalize_kernel(long n, const double* __restrict__ y0,
+                                 const double* __restrict__ y1, double* __restrict__ v0,
+                                 double* __restrict__ v1, double* out) {
   __shared__ double red[32];
+  const double* y = blockIdx.x == 0 ? y0 : y1;
+  double* v = blockIdx.x == 0 ? v0 : v1;
   double s = 0.0;
   for (long i = threadIdx.x; i < n; i += blockDim.x) s = fma(y[i], y[i], s);
   s = warp_sum(s);
@@ -116,7 +136,7 @@ __global__ void normalize_kernel(long n, const double* __restrict__ y, double* _
   const double nrm = sqrt(t);
   const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
   for (long i = threadIdx.x; i < n; i += blockDim.x) v[i] = y[i] * inv;
-  if (threadIdx.x == 0) *out = nrm;
+  if (threadIdx.x == 0) out[blockIdx.x] = nrm;
 }
 
 __global__ void delta_kernel(double* scal, long n) {
@@ -170,13 +190,9 @@ int refine_middle(long n, const double* S, double* R, double* lam, double* v0, d
   lambda_kernel<<<gblocks, threads, 0, st>>>(n, S, n, R, n, lam, v0, v1, scal);
   EVD_LAUNCHED();
   for (int p = 0; p < kPowerSteps; ++p) {
-    symv_kernel<<<wblocks, threads, 0, st>>>(n, S, n, lam, v0, y0, 1);
+    symv_kernel<<<dim3(wblocks, 2), threads, 0, st>>>(n, S, R, n, lam, v0, v1, y0, y1);
     EVD_LAUNCHED();
-    normalize_kernel<<<1, 1024, 0, st>>>(n, y0, v0, scal + 4);
-    EVD_LAUNCHED();
-    symv_kernel<<<wblocks, threads, 0, st>>>(n, R, n, lam, v1, y1, 0);
-    EVD_LAUNCHED();
-    normalize_kernel<<<1, 1024, 0, st>>>(n, y1, v1, scal + 5);
+    normalize_kernel<<<2, 1024, 0, st>>>(n, y0, y1, v0, v1, scal + 4);
     EVD_LAUNCHED();
   }
   delta_kernel<<<1, 1, 0, st>>>(scal, n);
