@@ -142,6 +142,7 @@ __device__ __forceinline__ void load_tile(double* smem, GPtr g, SOff s_off, int 
 template <bool TA, bool TB, int BM, int BN, int BK, int WM, int WN, int STAGES, int MMA>
 __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32)
     dgemm_kernel(const GemmArgs p) {
+  pdl_entry(BN == 32);  // the skinny products
   constexpr int NWM = BM / WM, NWN = BN / WN;
   constexpr int NT = NWM * NWN * 32;
   // MMA: 0 = m8n8k4, 1 = m16n8k4, 2 = m16n8k8, 3 = m16n8k16
@@ -391,6 +392,7 @@ struct TileCopy {
 template <bool TA, bool TB, int BM, int BN, int BK, int WM, int WN, int STAGES, int MMA>
 __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32)
     dgemm_fast_kernel(const GemmArgs p) {
+  pdl_entry(BN == 32);
   constexpr int NWM = BM / WM, NWN = BN / WN;
   constexpr int NT = NWM * NWN * 32;
   constexpr int MR = (MMA >= 1) ? 16 : 8;
@@ -595,6 +597,7 @@ __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32)
 __global__ void dgemm_splitk_reduce_kernel(int m, int n, int splits, long batch_count,
                                            const double* ws, double alpha, double beta,
                                            double* C, long ldc, long sC) {
+  pdl_entry();
   long total = (long)m * n;
   for (long b = 0; b < batch_count; ++b) {
     const double* W = ws + b * splits * total;
@@ -621,8 +624,7 @@ int launch_cfg(GemmArgs p, int grid_x, int grid_y, cudaStream_t st) {
   auto kern = FAST ? dgemm_fast_kernel<TA, TB, BM, BN, BK, WM, WN, STAGES, MMA>
                    : dgemm_kernel<TA, TB, BM, BN, BK, WM, WN, STAGES, MMA>;
   EVD_TRY(smem_attr_once((const void*)kern, (int)smem));
-  kern<<<dim3(grid_x, grid_y), NT, smem, st>>>(p);
-  EVD_LAUNCHED();
+  EVD_TRY(launch_pdl(kern, dim3(grid_x, grid_y), NT, smem, st, p));
   return EVD_SUCCESS;
 }
 
@@ -692,9 +694,8 @@ static int gemm_run(GemmArgs p, bool ta, bool tb, long batch, cudaStream_t st,
   if (p.splitk > 1) {
     long total = (long)p.m * p.n;
     int blocks = (int)std::min<long>((total + 255) / 256, 4L * device_sm_count());
-    dgemm_splitk_reduce_kernel<<<blocks, 256, 0, st>>>(p.m, p.n, p.splitk, batch, p.ws,
-                                                       p.alpha, p.beta, p.C, p.ldc, p.sC);
-    EVD_LAUNCHED();
+    EVD_TRY(launch_pdl(dgemm_splitk_reduce_kernel, blocks, 256, 0, st, p.m, p.n, p.splitk, batch,
+                       p.ws, p.alpha, p.beta, p.C, p.ldc, p.sC));
   }
   return EVD_SUCCESS;
 }

@@ -215,6 +215,7 @@ __device__ void tile_factor(double* src, long ld, int mm, double* Rdst, long ldR
 __global__ void __launch_bounds__(kThreads, 1) tsqr_up_kernel(const TsqrPlan plan, double* A,
                                                               long lda, double* ws, double* Rout,
                                                               long ldr) {
+  pdl_entry();
   __shared__ TileSmem sm;
   __shared__ int is_last;
   int* cnt = reinterpret_cast<int*>(ws + plan.cnt_off);
@@ -316,6 +317,7 @@ __device__ __forceinline__ void back_solve(double (&x)[kNB], const double* Bt, c
 // reflectors in each node's tile): one CTA per node, Q = E - V K.
 __global__ void __launch_bounds__(kThreads, 1)
     tsqr_q_kernel(const TsqrPlan plan, double* A, long lda, double* ws) {
+  pdl_entry();
   extern __shared__ __align__(16) double q_smem[];
   QSmem& sm = *reinterpret_cast<QSmem*>(q_smem);
   int idx = blockIdx.x, level = 0;
@@ -481,6 +483,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tsqr_finish_kernel(const TsqrPlan plan, const double* ws, double* A, long lda, int mode,
                        double* Yout, long ldy, double* Wout, long ldw, const double* Rin,
                        long ldr, double* Aband, long ldband) {
+  pdl_entry();
   extern __shared__ __align__(16) double dsm[];
   FinishSmem& sm = *reinterpret_cast<FinishSmem*>(dsm);
   const int t = blockIdx.x;
@@ -639,15 +642,14 @@ int panel_qr_launch(long m, double* A, long lda, double* ws, int mode, double* Y
   TsqrPlan plan = make_plan(m);
   if (plan.nlev >= kMaxLevels) return EVD_ERR_INVALID_ARG;
   EVD_TRY(finish_attr());
-  tsqr_up_kernel<<<plan.T[0], kThreads, 0, st>>>(plan, A, lda, ws, R, ldr);
-  EVD_LAUNCHED();
+  EVD_TRY(launch_pdl(tsqr_up_kernel, plan.T[0], kThreads, 0, st, plan, A, lda, ws, R,
+                     ldr));
   int nodes = 0;
   for (int l = 0; l < plan.nlev; ++l) nodes += plan.T[l];
-  tsqr_q_kernel<<<nodes, kThreads, sizeof(QSmem), st>>>(plan, A, lda, ws);
-  EVD_LAUNCHED();
-  tsqr_finish_kernel<<<plan.T[0], kThreads, sizeof(FinishSmem), st>>>(
-      plan, ws, A, lda, mode, Yout, ldy, Wout, ldw, R, ldr, Aband, ldband);
-  EVD_LAUNCHED();
+  EVD_TRY(launch_pdl(tsqr_q_kernel, nodes, kThreads, sizeof(QSmem), st, plan, A, lda,
+                     ws));
+  EVD_TRY(launch_pdl(tsqr_finish_kernel, plan.T[0], kThreads, sizeof(FinishSmem), st,
+                     plan, ws, A, lda, mode, Yout, ldy, Wout, ldw, R, ldr, Aband, ldband));
   return EVD_SUCCESS;
 }
 

@@ -135,6 +135,7 @@ __global__ void absmax_kernel(long n, const double* d, const double* e, double* 
 // scaled copy + padding + tears at every leaf boundary
 __global__ void init_kernel(long n, long np, int s, const double* d, const double* e,
                             const double* scal, double* dw, double* ew) {
+  pdl_entry();
   const double nrm = scal[0];
   const double inv = (nrm > 0.0) ? 1.0 / nrm : 1.0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < np; i += (long)gridDim.x * blockDim.x) {
@@ -169,6 +170,7 @@ constexpr int kLeafWarps = 4;
 __global__ void __launch_bounds__(32 * kLeafWarps)
     leaf_ql_kernel(int s, int nleaves, double* dw, const double* ew, double* Zw, long ldz,
                    int* err) {
+  pdl_entry();
   __shared__ double zsm[kLeafWarps][kLeafMax * 32];
   const unsigned all = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -278,6 +280,7 @@ struct LevelArgs {
 
 // z vector, rho and the merged sort order.  grid (ceil(N/256), nm)
 __global__ void merge_setup_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.y;
   const long lo = (long)m * a.N, mid = lo + a.n1;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -344,6 +347,7 @@ __device__ __forceinline__ int block_prefix(bool flag, int* s_cnt, int* total) {
 }
 
 __global__ void __launch_bounds__(kDefMax) merge_deflate_kernel(LevelArgs a) {
+  pdl_entry();
   // entry 0 is the survivor pending from the previous chunk, entry 1 + i the
   // chunk's element i
   __shared__ double s_d[kDefMax + 1], s_z[kDefMax + 1];
@@ -578,6 +582,7 @@ __global__ void __launch_bounds__(kDefMax) merge_deflate_kernel(LevelArgs a) {
 
 // Apply the recorded rotations to the block's columns; thread = row.
 __global__ void merge_rotate_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.y;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= a.N) return;
@@ -610,6 +615,7 @@ int col_chunk(int N, int cols, int nm) {
 }
 
 __global__ void merge_gather_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.z;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= a.N) return;
@@ -649,6 +655,7 @@ __global__ void merge_gather_kernel(LevelArgs a) {
 // merge GEMMs, which write Zn[:, 0:Kmax] for every merge of the level.
 // grid (ceil(N/256), ceil(N/chunk), nm).
 __global__ void merge_copy_deflated_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.z;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= a.N) return;
@@ -779,6 +786,7 @@ __device__ void secular_root_warp(int K, int j, const double* dK, const double* 
 
 // grid (ceil(Kmax*32/256), nm), block 256: one warp per root
 __global__ void merge_secular_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.y;
   const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long lo = (long)m * a.N;
@@ -797,6 +805,7 @@ __global__ void merge_secular_kernel(LevelArgs a) {
 // One warp per i; each lane keeps its partial product as mantissa * 2^e so
 // that no partial product over- or underflows.
 __global__ void merge_loewner_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.y;
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -832,6 +841,7 @@ __global__ void merge_loewner_kernel(LevelArgs a) {
 // U(:, j): v_i = zhat_i / (d_i - lambda_j), normalised; rows placed in the
 // type order of Ut (types 1,2) and Ub (types 2,3).  grid (Kmax, nm), block 256.
 __global__ void merge_vectors_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.y;
   const int j = blockIdx.x;
   const long lo = (long)m * a.N;
@@ -877,6 +887,7 @@ __global__ void merge_vectors_kernel(LevelArgs a) {
 // Final ascending order of the merged eigenvalues and scatter of the vectors
 // back into Zw[lo:hi, lo:hi].  grid (ceil(N/256), nm): thread = output source.
 __global__ void merge_finalize_rank_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.y;
   const int q = blockIdx.x * blockDim.x + threadIdx.x;  // source index: roots then deflated
   if (q >= a.N) return;
@@ -915,6 +926,7 @@ __global__ void merge_finalize_rank_kernel(LevelArgs a) {
 // Zw[lo:hi, lo + p] = Zn[:, perm[p]], dw[lo + p] = sorted value.
 // grid (ceil(N/256), ceil(N/chunk), nm): thread = row, blockIdx.y = columns.
 __global__ void merge_scatter_kernel(LevelArgs a) {
+  pdl_entry();
   const int m = blockIdx.z;
   const int p0 = blockIdx.y * a.chunk;
   const long lo = (long)m * a.N;
@@ -999,13 +1011,12 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
   double* dw = work + P.o_d;
   double* ew = work + P.o_e;
   double* Zw = work + P.o_Z;
-  init_kernel<<<ceil_div_i(np, 256), 256, 0, st>>>(n, np, P.s, d, e, scal, dw, ew);
-  EVD_LAUNCHED();
+  EVD_TRY(launch_pdl(init_kernel, ceil_div_i(np, 256), 256, 0, st,
+                     n, np, P.s, d, e, scal, dw, ew));
   EVD_CUDA_TRY(cudaMemsetAsync(Zw, 0, sizeof(double) * np * np, st));
   const int nleaves = 1 << P.L;
-  leaf_ql_kernel<<<ceil_div_i(nleaves, kLeafWarps), 32 * kLeafWarps, 0, st>>>(
-      P.s, nleaves, dw, ew, Zw, np, err);
-  EVD_LAUNCHED();
+  EVD_TRY(launch_pdl(leaf_ql_kernel, ceil_div_i(nleaves, kLeafWarps), 32 * kLeafWarps, 0, st,
+                     P.s, nleaves, dw, ew, Zw, np, err));
 
   std::vector<int> hdesc;
   for (int lev = 1; lev <= P.L; ++lev) {
@@ -1047,10 +1058,8 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
     a.Ub = work + P.o_Ub;
     a.Zn = work + P.o_Zn;
     dim3 gN(ceil_div_i(a.N, 256), a.nm);
-    merge_setup_kernel<<<gN, 256, 0, st>>>(a);
-    EVD_LAUNCHED();
-    merge_deflate_kernel<<<a.nm, std::min(kDefMax, (a.N + 31) / 32 * 32), 0, st>>>(a);
-    EVD_LAUNCHED();
+    EVD_TRY(launch_pdl(merge_setup_kernel, gN, 256, 0, st, a));
+    EVD_TRY(launch_pdl(merge_deflate_kernel, a.nm, std::min(kDefMax, (a.N + 31) / 32 * 32), 0, st, a));
     hdesc.resize(8 * a.nm);
     EVD_CUDA_TRY(cudaMemcpyAsync(hdesc.data(), a.desc, sizeof(int) * 8 * a.nm,
                                  cudaMemcpyDeviceToHost, st));
@@ -1070,26 +1079,21 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
     a.K12max = (K12 + 1) & ~1;
     a.K23max = (K23 + 1) & ~1;
     if (nrmax > 0) {
-      merge_rotate_kernel<<<gN, 256, 0, st>>>(a);
-      EVD_LAUNCHED();
+      EVD_TRY(launch_pdl(merge_rotate_kernel, gN, 256, 0, st, a));
     }
     {
       const int cols = std::max(Kmax, std::max(a.K12max, a.K23max));
       if (cols > 0) {
         a.chunk = col_chunk(a.N, cols, a.nm);
         dim3 gG(ceil_div_i(a.N, 256), ceil_div_i(cols, a.chunk), a.nm);
-        merge_gather_kernel<<<gG, 256, 0, st>>>(a);
-        EVD_LAUNCHED();
+        EVD_TRY(launch_pdl(merge_gather_kernel, gG, 256, 0, st, a));
       }
     }
     if (Kmax > 0) {
       dim3 gK(ceil_div_i((long)Kmax * 32, 256), a.nm);
-      merge_secular_kernel<<<gK, 256, 0, st>>>(a);
-      EVD_LAUNCHED();
-      merge_loewner_kernel<<<gK, 256, 0, st>>>(a);
-      EVD_LAUNCHED();
-      merge_vectors_kernel<<<dim3(Kmax, a.nm), 256, 0, st>>>(a);
-      EVD_LAUNCHED();
+      EVD_TRY(launch_pdl(merge_secular_kernel, gK, 256, 0, st, a));
+      EVD_TRY(launch_pdl(merge_loewner_kernel, gK, 256, 0, st, a));
+      EVD_TRY(launch_pdl(merge_vectors_kernel, dim3(Kmax, a.nm), 256, 0, st, a));
       // Zn[0:n1, 0:Kmax] = Qt Ut ; Zn[n1:N, 0:Kmax] = Qb Ub   (batched over merges)
       const long sZ = (long)a.N * a.N;
       const bool emul = oz && (double)a.n1 * Kmax * std::max(K12, K23) >= kOzMergeMin;
@@ -1131,12 +1135,9 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
     }
     a.chunk = col_chunk(a.N, a.N, a.nm);
     dim3 gC(ceil_div_i(a.N, 256), ceil_div_i(a.N, a.chunk), a.nm);
-    merge_copy_deflated_kernel<<<gC, 256, 0, st>>>(a);
-    EVD_LAUNCHED();
-    merge_finalize_rank_kernel<<<gN, 256, 0, st>>>(a);
-    EVD_LAUNCHED();
-    merge_scatter_kernel<<<gC, 256, 0, st>>>(a);
-    EVD_LAUNCHED();
+    EVD_TRY(launch_pdl(merge_copy_deflated_kernel, gC, 256, 0, st, a));
+    EVD_TRY(launch_pdl(merge_finalize_rank_kernel, gN, 256, 0, st, a));
+    EVD_TRY(launch_pdl(merge_scatter_kernel, gC, 256, 0, st, a));
   }
   dim3 gf(ceil_div_i(n, 256), (unsigned)std::min<long>(n, 65535));
   if (out_after) EVD_CUDA_TRY(cudaStreamWaitEvent(st, out_after, 0));

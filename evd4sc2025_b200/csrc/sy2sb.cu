@@ -32,6 +32,7 @@ namespace {
 
 __global__ void copy_block_kernel(long m, long n, const double* __restrict__ src, long lds,
                                   double* __restrict__ dst, long ldd) {
+  pdl_entry();
   for (long j = blockIdx.y; j < n; j += gridDim.y)
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < m;
          i += (long)gridDim.x * blockDim.x)
@@ -108,9 +109,8 @@ int sy2sb(long M, long N, long b, long nb, double* OA, long ldOA, double* dA, lo
     if (off > 0) {
       // this frame's first nb columns of the updated trailing matrix -> dA
       dim3 grid(ceil_div_i(Nf, 256), (unsigned)std::min<long>(nb, 65535));
-      copy_block_kernel<<<grid, 256, 0, st>>>(Nf, nb, OA + off + off * ldOA, ldOA,
-                                              dA + off + off * ldA, ldA);
-      EVD_LAUNCHED();
+      EVD_TRY(launch_pdl(copy_block_kernel, grid, 256, 0, st, Nf, nb, OA + off + off * ldOA,
+                         ldOA, dA + off + off * ldA, ldA));
     }
     for (long i = b; i <= nb && i < Nf; i += b) {
       const long m = Nf - i;
@@ -183,8 +183,7 @@ int copy_matrix(long m, long n, const double* src, long lds, double* dst, long l
                 cudaStream_t st) {
   if (m <= 0 || n <= 0) return EVD_SUCCESS;
   dim3 grid(ceil_div_i(m, 256), (unsigned)std::min<long>(n, 65535));
-  copy_block_kernel<<<grid, 256, 0, st>>>(m, n, src, lds, dst, ldd);
-  EVD_LAUNCHED();
+  EVD_TRY(launch_pdl(copy_block_kernel, grid, 256, 0, st, m, n, src, lds, dst, ldd));
   return EVD_SUCCESS;
 }
 
