@@ -11,10 +11,10 @@
 //    shape is kept on purpose: the signs of R (hence of Y, W and the band)
 //    follow from the Householder sign rule applied node by node, so another
 //    tree gives R up to row signs, not the reference's R.  It runs as ONE
-//    up-sweep kernel: each CTA factors its tile in registers, publishes its R,
-//    and the last child to arrive at a parent (atomic counter) goes on to
-//    factor the parent.  Nobody waits, so there is no grid barrier and no
-//    spin.  The reference launches one kernel plus batched GEMMs per level.
+//    up-sweep kernel, a CTA per tree node, in which the columns of R stream up
+//    the tree: a parent works on a group of columns as soon as its children
+//    have published theirs, so all levels work at once.  The reference
+//    launches one kernel plus batched GEMMs per level.
 //  * tsqr_q_kernel forms the explicit thin Q of all nodes at once from their
 //    reflectors V (128 x 32, every tau = 1): Q_node = E - V K, E = [I; 0],
 //    K = T V_top^T, T^-1 = I + striu(V^T V): a Gram matrix on DMMA, one
@@ -39,7 +39,7 @@ namespace {
 constexpr int kTile = 128;        // rows per TSQR tile (reference: M = 128)
 constexpr int kNB = 32;           // panel width (reference: N = 32)
 constexpr int kFan = kTile / kNB; // children per tree node (their R factors fill one tile)
-constexpr int kThreads = 256;     // up-sweep: 8 warps x 4 columns
+constexpr int kThreads = 256;
 constexpr int kMaxLevels = 16;
 
 struct TsqrPlan {
@@ -70,13 +70,13 @@ TsqrPlan make_plan(long m) {
     ++L;
   }
   p.nlev = L + 1;
-  p.ncnt = coff;
+  p.ncnt = 1 + kNB / 8 * coff;  // the ticket, a counter per inner node and column group
   // Arrival counters come first, at a fixed offset: a workspace sized (and
   // zeroed) for the largest panel then serves every smaller panel, whose
   // counters are a prefix of the same region (the kernels reset each counter
   // after use).
   p.cnt_off = 0;
-  long off = (coff + 1) / 2 + 2;  // ints packed two per double
+  long off = (p.ncnt + 1) / 2 + 2;  // ints packed two per double
   off = (off + 1) / 2 * 2;        // keep the stacks 16-byte aligned
   for (int l = 1; l < p.nlev; ++l) {
     p.soff[l] = off;
@@ -86,179 +86,6 @@ TsqrPlan make_plan(long m) {
   off += kNB * kNB;
   p.total = off;
   return p;
-}
-
-// Householder QR of one tile (mm <= 128 rows, 32 columns) held in registers:
-// warp w owns columns w, w + 8, w + 16, w + 24, eight lanes per column (lane
-// group q = lane / 8 has column 8 q + w), and lane g of a group the 16 rows
-// 16 (e / 2) + 2 g + e % 2.  Writes R (32 x 32, upper; diag = -sign(x0) ||x||)
-// to Rdst and leaves the reflectors in the tile (column j, zero above row j).
-// Same steps as my_hou_kernel<128,32> (util/inc/kernelQR.h:215-414):
-// u = x/||x||, u0 += sign(u0), u scaled to ||u||^2 = 2.
-//
-// What bounds it: the chain of 32 columns.  Step j starts from the bare column
-// x in shared memory, and x^T a_c of every column and ||x||^2 (each group its
-// own copy) are reduced together; u^T a_c = s x^T a_c follows from the norm, so
-// a column costs one reduction, two reciprocal roots and one CTA barrier, where
-// a dot product with the finished reflector and then the norm took two
-// reductions in a row.  Branches are per warp (lane-wise ones cost more than
-// the work they skip); four warps with four lanes per column were slower.
-struct TileSmem {
-  __align__(16) double x[2][kTile];  // column j below row j (zero elsewhere)
-  double x0[2];                      // its row j
-  double RR[kNB];
-};
-
-// Sums over groups of eight lanes, two at a time.
-__device__ __forceinline__ void sum8x2(double& u, double& v) {
-#pragma unroll
-  for (int m = 4; m > 0; m >>= 1) {
-    const double a = __shfl_xor_sync(0xffffffffu, u, m);
-    const double b = __shfl_xor_sync(0xffffffffu, v, m);
-    u += a;
-    v += b;
-  }
-}
-__device__ void tile_factor(double* src, long ld, int mm, double* Rdst, long ldR, TileSmem& sm) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane & 7, col = 8 * (lane >> 3) + warp;
-  constexpr int kE = kTile / 8;  // rows per lane
-  constexpr int kTop = kNB / 8;  // of them in the first 32 rows
-  auto row_of = [&](int e) { return 16 * (e >> 1) + 2 * g + (e & 1); };
-  double a[kE];
-#pragma unroll
-  for (int e = 0; e < kE; ++e)
-    a[e] = (row_of(e) < mm) ? __ldcg(src + row_of(e) + (long)col * ld) : 0.0;
-
-  // column j to shared memory by the eight lanes that own it
-  auto publish = [&](int j) {
-    double2* x = reinterpret_cast<double2*>(sm.x[j & 1]);
-#pragma unroll
-    for (int e = 0; e < kE; e += 2) {
-      const int row = row_of(e);  // rows of e >= kTop are all below row j
-      x[row >> 1] = make_double2(e >= kTop || row > j ? a[e] : 0.0,
-                                 e >= kTop || row + 1 > j ? a[e + 1] : 0.0);
-      if (e < kTop) {
-        if (row == j) sm.x0[j & 1] = a[e];
-        if (row + 1 == j) sm.x0[j & 1] = a[e + 1];
-      }
-    }
-  };
-  if (col == 0) publish(0);
-  __syncthreads();
-#pragma unroll 1
-  for (int j = 0; j < kNB; ++j) {
-    double x[kE], d0 = 0.0, d1 = 0.0, n0 = 0.0, n1 = 0.0;
-    const double2* xs = reinterpret_cast<const double2*>(sm.x[j & 1]);
-    const double x0 = sm.x0[j & 1];
-#pragma unroll
-    for (int e = 0; e < kE; e += 2) {
-      const double2 v = xs[row_of(e) >> 1];
-      x[e] = v.x;
-      x[e + 1] = v.y;
-      n0 = fma(v.x, v.x, n0);
-      n1 = fma(v.y, v.y, n1);
-      d0 = fma(v.x, a[e], d0);
-      d1 = fma(v.y, a[e + 1], d1);
-    }
-    // this column's row j: lane (j / 2) % 8 of the group, e = 2 (j / 16) + j % 2
-    const double e0 = (j & 1) ? a[1] : a[0], e1 = (j & 1) ? a[3] : a[2];
-    const double aj = __shfl_sync(0xffffffffu, (j & 16) ? e1 : e0, (lane & 24) | ((j >> 1) & 7));
-    double nrm2 = n0 + n1, dot = d0 + d1;
-    sum8x2(nrm2, dot);
-    nrm2 = fma(x0, x0, nrm2);
-    // A zero column (nothing to annihilate) gets u = sqrt(2) e_j rather than
-    // u = 0: H = I - u u^T then only flips row j, R_jj = 0, every reflector
-    // keeps ||u||^2 = 2, and I - Q stays nonsingular for the Householder
-    // reconstruction (u = 0 would give a zero pivot there).
-    const bool live = nrm2 > 0.0;
-    const double rn = live ? rsqrt(nrm2) : 0.0;  // 1 / ||x||
-    const double c0 = x0 * rn;
-    const double sg = (c0 >= 0.0) ? 1.0 : -1.0;
-    const double c0n = c0 + sg;
-    const double s2 = rsqrt(fabs(c0n));
-    const double sc = rn * s2;                               // u = sc x below row j
-    const double u0 = live ? c0n * s2 : 1.4142135623730951;  // u in row j
-    const double d = (col > j) ? fma(sc, dot, u0 * aj) : 0.0;  // u^T a
-    const double f = -d * sc, fj = -d * u0;
-#pragma unroll
-    for (int e = 0; e < kTop; ++e) a[e] += (row_of(e) == j) ? fj : 0.0;
-#pragma unroll
-    for (int e = 0; e < kE; ++e) a[e] = fma(f, x[e], a[e]);
-    if (warp == ((j + 1) & 7) && j + 1 < kNB) {
-      if (col == j + 1) publish(j + 1);
-    }
-    if (warp == (j & 7)) {  // column j itself: its reflector
-      const bool mine = col == j;
-#pragma unroll
-      for (int e = 0; e < kE; ++e)
-        a[e] = (mine && (e >= kTop || row_of(e) > j)) ? sc * x[e] : a[e];
-#pragma unroll
-      for (int e = 0; e < kTop; ++e) a[e] = (mine && row_of(e) == j) ? u0 : a[e];
-      if (lane == 0) sm.RR[j] = -sg * (nrm2 * rn);
-    }
-    __syncthreads();
-  }
-
-  // R from the rows above the diagonal; reflectors back into the tile
-#pragma unroll
-  for (int e = 0; e < kE; ++e) {
-    const int row = row_of(e);
-    if (e < kTop) {
-      Rdst[row + (long)col * ldR] = (row < col) ? a[e] : ((row == col) ? sm.RR[col] : 0.0);
-      if (row < col) a[e] = 0.0;
-    }
-    if (row < mm) src[row + (long)col * ld] = a[e];
-  }
-}
-
-__global__ void __launch_bounds__(kThreads, 1) tsqr_up_kernel(const TsqrPlan plan, double* A,
-                                                              long lda, double* ws, double* Rout,
-                                                              long ldr) {
-  pdl_entry();
-  __shared__ TileSmem sm;
-  __shared__ int is_last;
-  int* cnt = reinterpret_cast<int*>(ws + plan.cnt_off);
-  int level = 0, idx = blockIdx.x;
-  for (;;) {
-    double* src;
-    long ld;
-    if (level == 0) {
-      src = A + (long)idx * kTile;
-      ld = lda;
-    } else {
-      src = ws + plan.soff[level] + (long)idx * kTile;
-      ld = plan.rows[level];
-    }
-    int mm = min(kTile, plan.rows[level] - idx * kTile);
-    const bool root = (plan.T[level] == 1);
-    double* Rdst;
-    long ldR;
-    if (root) {
-      Rdst = Rout;
-      ldR = ldr;
-    } else {
-      Rdst = ws + plan.soff[level + 1] + (long)idx * kNB;
-      ldR = plan.rows[level + 1];
-    }
-    tile_factor(src, ld, mm, Rdst, ldR, sm);
-    if (root) break;
-    const int parent = idx / kFan;
-    const int nch = min(kFan, plan.T[level] - kFan * parent);
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int* c = cnt + plan.coff[level + 1] + parent;
-      int old = atomicAdd(c, 1);
-      is_last = (old == nch - 1);
-      if (is_last) *c = 0;  // self-reset for the next panel
-    }
-    __syncthreads();
-    if (!is_last) break;
-    __threadfence();
-    ++level;
-    idx = parent;
-  }
 }
 
 // ---- 32-wide products on the FP64 tensor pipe ----
@@ -285,6 +112,296 @@ __device__ __forceinline__ void row_block(const double* A, const double* B, int 
 #pragma unroll
     for (int ni = 0; ni < 4; ++ni) mma8(d[ni], af, B[(4 * kk + t) * kLd + 8 * ni + g]);
   }
+}
+
+// ---- up-sweep: all tree nodes at once, columns streamed up the tree ----
+// One CTA per node (128 x 32 tile: rows of the panel, or the stacked R factors
+// of four children).  A column of R is final as soon as its reflector is, and a
+// parent needs of its children only the columns up to the one it works on, so
+// a node takes its columns in four groups of eight, each as soon as all children
+// have published theirs: load, apply the node's earlier reflectors as one
+// compact-WY update on DMMA (A -= V T^T V^T A), factor the eight columns, publish
+// their part of R, extend T.  All levels work at the same time, one group
+// behind each other.  Same steps per column as my_hou_kernel<128,32>
+// (util/inc/kernelQR.h:215-414): u = x/||x||, u0 += sign(u0), u scaled to
+// ||u||^2 = 2; diag(R) = -sign(x0) ||x||.
+//
+// What bounds it: the chain of 32 columns, about 600 cycles each, once, plus
+// eight columns per further level; factoring a level after the other took 21 us
+// per level.  In the eight columns a warp owns one column, a lane four rows;
+// x^T a and ||x||^2 are reduced together from the bare column x, and u^T a
+// follows from the norm.
+//
+// Progress: CTAs take nodes from a ticket, leaves first, and wait only for
+// children, which earlier tickets own.  A wait that outlasts 4 s fills the
+// node's R with NaN, which the tridiagonal solver rejects.
+constexpr int kGrp = 8, kGroups = kNB / kGrp;
+constexpr int kWLd = kGrp + 4;  // row stride of 8-wide matrices (conflict-free fragments)
+
+struct UpSmem {
+  double V[kNB * kVLd];
+  double A[kGrp * kVLd];
+  double T[kNB * kLd];
+  double W[2][kNB * kWLd], W2[kNB * kWLd];
+  double x[2][kTile];  // column j below row j (zero elsewhere)
+  double x0[2];        // its row j
+  double RR[kNB];
+  int node, ok;
+};
+
+// D (8 x 8 tile) += A B over k-steps [k0, k1) in two chains; a(kk), b(kk) give
+// this lane's fragment elements.
+template <typename FA, typename FB>
+__device__ __forceinline__ void tile_mma(double (&d)[2], int k0, int k1, FA a, FB b) {
+  double e[2] = {0.0, 0.0};
+  for (int kk = k0; kk < k1; kk += 2) {
+    mma8(d, a(kk), b(kk));
+    mma8(e, a(kk + 1), b(kk + 1));
+  }
+  d[0] += e[0];
+  d[1] += e[1];
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    tsqr_up_kernel(const TsqrPlan plan, double* A, long lda, double* ws, double* Rout, long ldr) {
+  pdl_entry();
+  extern __shared__ __align__(16) double up_smem[];
+  UpSmem& sm = *reinterpret_cast<UpSmem*>(up_smem);
+  int* ticket = reinterpret_cast<int*>(ws + plan.cnt_off);
+  int* cnt = ticket + 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  if (tid == 0) {
+    sm.node = atomicAdd(ticket, 1);
+    sm.ok = 1;
+  }
+  for (int e = tid; e < kNB * kLd; e += kThreads) sm.T[e] = 0.0;
+  __syncthreads();
+  int idx = sm.node, level = 0;
+  while (idx >= plan.T[level]) idx -= plan.T[level++];
+  const bool root = plan.T[level] == 1;
+  double* src = (level == 0) ? A + (long)idx * kTile : ws + plan.soff[level] + (long)idx * kTile;
+  const long ld = (level == 0) ? lda : plan.rows[level];
+  const int mm = min(kTile, plan.rows[level] - idx * kTile);
+  double* Rdst = root ? Rout : ws + plan.soff[level + 1] + (long)idx * kNB;
+  const long ldR = root ? ldr : plan.rows[level + 1];
+  const int nch = level ? min(kFan, plan.T[level - 1] - kFan * idx) : 0;
+  int* arrived = level ? cnt + (plan.coff[level] + idx) * kGroups : nullptr;
+  int* up = root ? nullptr : cnt + (plan.coff[level + 1] + idx / kFan) * kGroups;
+
+  // element e of a thread's share of a group: row tid % 128, columns tid / 128 + 2 e
+  const int lr = tid & (kTile - 1), lc = tid >> 7;
+  double nxt[4];
+  auto fetch = [&](int G) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      nxt[e] = (lr < mm) ? __ldcg(src + lr + (long)(kGrp * G + lc + 2 * e) * ld) : 0.0;
+  };
+  if (level == 0) fetch(0);
+
+#pragma unroll 1
+  for (int G = 0; G < kGroups; ++G) {
+    if (level > 0) {
+      if (tid == 0) {
+        int* f = arrived + G;
+        unsigned long long t0 = 0, now;
+        for (unsigned it = 1; sm.ok && ld_acquire(f) < nch; ++it) {
+          if ((it & 1023u) != 0) continue;
+          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+          if (t0 == 0) t0 = now;
+          if (now - t0 > 4000000000ull) {
+            sm.ok = 0;
+            break;
+          }
+        }
+        *f = 0;  // ready for the next panel
+      }
+      __syncthreads();
+      fetch(G);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      sm.A[(lc + 2 * e) * kVLd + lr] = sm.ok ? nxt[e] : __longlong_as_double(0x7ff8000000000000ll);
+    if (level == 0 && G + 1 < kGroups) fetch(G + 1);
+    __syncthreads();
+    if (G > 0) {
+      // W = V^T A: tile warp / 2, half of K per warp
+      if (warp < 2 * G) {
+        const int mi = warp >> 1, h = warp & 1;
+        double d[2] = {0.0, 0.0};
+        const double* va = sm.V + (8 * mi + g) * kVLd + t;
+        const double* ab = sm.A + g * kVLd + t;
+        tile_mma(d, 16 * h, 16 * h + 16, [&](int kk) { return va[4 * kk]; },
+                 [&](int kk) { return ab[4 * kk]; });
+        sm.W[h][(8 * mi + g) * kWLd + 2 * t] = d[0];
+        sm.W[h][(8 * mi + g) * kWLd + 2 * t + 1] = d[1];
+      }
+      __syncthreads();
+      if (warp < G) {  // W2 = T^T W
+        double d[2] = {0.0, 0.0};
+        tile_mma(d, 0, 2 * G, [&](int kk) { return sm.T[(4 * kk + t) * kLd + 8 * warp + g]; },
+                 [&](int kk) {
+                   return sm.W[0][(4 * kk + t) * kWLd + g] + sm.W[1][(4 * kk + t) * kWLd + g];
+                 });
+        sm.W2[(8 * warp + g) * kWLd + 2 * t] = d[0];
+        sm.W2[(8 * warp + g) * kWLd + 2 * t + 1] = d[1];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {  // A -= V W2
+        const int row = 8 * (2 * warp + q) + g;
+        double d[2] = {0.0, 0.0};
+        tile_mma(d, 0, 2 * G, [&](int kk) { return sm.V[(4 * kk + t) * kVLd + row]; },
+                 [&](int kk) { return sm.W2[(4 * kk + t) * kWLd + g]; });
+        sm.A[(2 * t) * kVLd + row] -= d[0];
+        sm.A[(2 * t + 1) * kVLd + row] -= d[1];
+      }
+      __syncthreads();
+    }
+    // ---- the eight columns: warp w has column 8 G + w, lane l rows 4 l .. 4 l + 3
+    const int col = kGrp * G + warp;
+    double a[4];
+    {
+      const double2 p = *reinterpret_cast<const double2*>(sm.A + warp * kVLd + 4 * lane);
+      const double2 q = *reinterpret_cast<const double2*>(sm.A + warp * kVLd + 4 * lane + 2);
+      a[0] = p.x;
+      a[1] = p.y;
+      a[2] = q.x;
+      a[3] = q.y;
+    }
+    auto publish = [&](int j) {  // this warp's column j to shared memory
+      double2* x = reinterpret_cast<double2*>(sm.x[j & 1] + 4 * lane);
+      const int r = 4 * lane;
+      x[0] = make_double2(r > j ? a[0] : 0.0, r + 1 > j ? a[1] : 0.0);
+      x[1] = make_double2(r + 2 > j ? a[2] : 0.0, r + 3 > j ? a[3] : 0.0);
+      if (lane == (j >> 2)) {
+        const double lo = (j & 1) ? a[1] : a[0], hi = (j & 1) ? a[3] : a[2];
+        sm.x0[j & 1] = (j & 2) ? hi : lo;
+      }
+    };
+    if (warp == 0) publish(kGrp * G);
+    __syncthreads();
+#pragma unroll 1
+    for (int w = 0; w < kGrp; ++w) {
+      const int j = kGrp * G + w;
+      const double x0 = sm.x0[j & 1];
+      const double2 p = *reinterpret_cast<const double2*>(sm.x[j & 1] + 4 * lane);
+      const double2 q = *reinterpret_cast<const double2*>(sm.x[j & 1] + 4 * lane + 2);
+      double nrm2 = fma(p.x, p.x, p.y * p.y) + fma(q.x, q.x, q.y * q.y);
+      double dot = fma(p.x, a[0], p.y * a[1]) + fma(q.x, a[2], q.y * a[3]);
+      const double lo = (j & 1) ? a[1] : a[0], hi = (j & 1) ? a[3] : a[2];
+      const double aj = __shfl_sync(0xffffffffu, (j & 2) ? hi : lo, j >> 2);
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) {
+        const double u = __shfl_xor_sync(0xffffffffu, nrm2, m);
+        const double v = __shfl_xor_sync(0xffffffffu, dot, m);
+        nrm2 += u;
+        dot += v;
+      }
+      nrm2 = fma(x0, x0, nrm2);
+      // A zero column (nothing to annihilate) gets u = sqrt(2) e_j rather than
+      // u = 0: H = I - u u^T then only flips row j, R_jj = 0, every reflector
+      // keeps ||u||^2 = 2, and I - Q stays nonsingular for the Householder
+      // reconstruction (u = 0 would give a zero pivot there).
+      const bool live = nrm2 > 0.0;
+      const double rn = live ? rsqrt(nrm2) : 0.0;  // 1 / ||x||
+      const double c0 = x0 * rn;
+      const double sg = (c0 >= 0.0) ? 1.0 : -1.0;
+      const double c0n = c0 + sg;
+      const double s2 = rsqrt(fabs(c0n));
+      const double sc = rn * s2;                               // u = sc x below row j
+      const double u0 = live ? c0n * s2 : 1.4142135623730951;  // u in row j
+      const bool at = lane == (j >> 2);
+      if (warp > w) {
+        const double d = fma(sc, dot, u0 * aj);  // u^T a
+        const double f = -d * sc, fj = -d * u0;
+        a[0] = fma(f, p.x, a[0]) + ((at && (j & 3) == 0) ? fj : 0.0);
+        a[1] = fma(f, p.y, a[1]) + ((at && (j & 3) == 1) ? fj : 0.0);
+        a[2] = fma(f, q.x, a[2]) + ((at && (j & 3) == 2) ? fj : 0.0);
+        a[3] = fma(f, q.y, a[3]) + ((at && (j & 3) == 3) ? fj : 0.0);
+        if (warp == w + 1) publish(j + 1);
+      } else if (warp == w) {
+        const double x[4] = {p.x, p.y, q.x, q.y};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          a[i] = (4 * lane + i > j) ? sc * x[i] : a[i];
+          a[i] = (at && (j & 3) == i) ? u0 : a[i];
+        }
+        if (lane == 0) sm.RR[j] = -sg * (nrm2 * rn);
+      }
+      __syncthreads();
+    }
+    // ---- R of these columns to the parent, reflectors to V and the tile
+    if (lane < kNB / 4) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = 4 * lane + i;
+        Rdst[row + (long)col * ldR] = (row < col) ? a[i] : ((row == col) ? sm.RR[col] : 0.0);
+      }
+    }
+    if (up != nullptr) {
+      __syncthreads();
+      if (tid == 0) {
+        __threadfence();
+        atomicAdd(up + G, 1);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = 4 * lane + i;
+      const double v = (row >= col) ? a[i] : 0.0;
+      sm.V[col * kVLd + row] = v;
+      if (row < mm) src[row + (long)col * ld] = v;
+    }
+    if (G + 1 == kGroups) break;
+    __syncthreads();
+    // ---- T: its new columns are T22 = (I + striu(V2^T V2))^-1 and
+    // T12 = -T11 (V1^T V2) T22
+    if (warp < 2 * (G + 1)) {
+      const int mi = warp >> 1, h = warp & 1;
+      double d[2] = {0.0, 0.0};
+      const double* va = sm.V + (8 * mi + g) * kVLd + t;
+      const double* vb = sm.V + (8 * G + g) * kVLd + t;
+      tile_mma(d, 16 * h, 16 * h + 16, [&](int kk) { return va[4 * kk]; },
+               [&](int kk) { return vb[4 * kk]; });
+      sm.W[h][(8 * mi + g) * kWLd + 2 * t] = d[0];
+      sm.W[h][(8 * mi + g) * kWLd + 2 * t + 1] = d[1];
+    }
+    __syncthreads();
+    if (warp == 0 && lane < kGrp) {  // column `lane` of T22, from its bottom
+      double c[kGrp];
+#pragma unroll
+      for (int i = kGrp - 1; i >= 0; --i) {
+        double acc = 0.0;
+#pragma unroll
+        for (int k = i + 1; k < kGrp; ++k)
+          acc = fma(sm.W[0][(8 * G + i) * kWLd + k] + sm.W[1][(8 * G + i) * kWLd + k], c[k], acc);
+        c[i] = (i < lane) ? -acc : (i == lane ? 1.0 : 0.0);
+        sm.T[(8 * G + i) * kLd + 8 * G + lane] = c[i];
+      }
+    }
+    __syncthreads();
+    if (warp < G) {  // P = (V1^T V2) T22
+      double d[2] = {0.0, 0.0};
+      tile_mma(d, 0, 2,
+               [&](int kk) {
+                 const int at = (8 * warp + g) * kWLd + 4 * kk + t;
+                 return sm.W[0][at] + sm.W[1][at];
+               },
+               [&](int kk) { return sm.T[(8 * G + 4 * kk + t) * kLd + 8 * G + g]; });
+      sm.W2[(8 * warp + g) * kWLd + 2 * t] = d[0];
+      sm.W2[(8 * warp + g) * kWLd + 2 * t + 1] = d[1];
+    }
+    __syncthreads();
+    if (warp < G) {  // T12 = -T11 P
+      double d[2] = {0.0, 0.0};
+      tile_mma(d, 0, 2 * G, [&](int kk) { return sm.T[(8 * warp + g) * kLd + 4 * kk + t]; },
+               [&](int kk) { return sm.W2[(4 * kk + t) * kWLd + g]; });
+      sm.T[(8 * warp + g) * kLd + 8 * G + 2 * t] = -d[0];
+      sm.T[(8 * warp + g) * kLd + 8 * G + 2 * t + 1] = -d[1];
+    }
+    // T and V are next read after the barriers of the next group's load
+  }
+  if (root && tid == 0) *ticket = 0;  // every node has been taken: ready for the next panel
 }
 
 struct QSmem {
@@ -610,6 +727,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 int finish_attr() {
   EVD_TRY(smem_attr_once((const void*)tsqr_finish_kernel, (int)sizeof(FinishSmem)));
+  EVD_TRY(smem_attr_once((const void*)tsqr_up_kernel, (int)sizeof(UpSmem)));
   EVD_TRY(smem_attr_once((const void*)tsqr_q_kernel, (int)sizeof(QSmem)));
   return EVD_SUCCESS;
 }
@@ -631,21 +749,21 @@ int panel_counters_reset(long m, double* ws, cudaStream_t st) {
   return EVD_SUCCESS;
 }
 
-// Three launches.  Measured on B200, us per panel, before (explicit node Q's by
-// 32 rank-1 updates, dot products after finished reflectors, row-by-row solves)
-// -> now: m = 128 89 -> 47, 992 178 -> 93, 4096 235 -> 119, 16384 226 -> 148.
-// What is left: 21 us per tree level (32 dependent columns), then 6 us for the
-// node Q's and 16 us to finish, half of it the 32 steps of the LU.
+// Three launches.  Measured on B200, us per panel, with a tree level after the
+// other, explicit node Q's by 32 rank-1 updates and row-by-row solves -> now:
+// m = 128 89 -> 48, 992 178 -> 65, 4096 235 -> 72, 16384 226 -> 95.  What is left:
+// the 32 dependent columns, 5 us per further tree level, 6 us for the node Q's
+// and 16 us to finish, half of it the 32 steps of the LU.
 int panel_qr_launch(long m, double* A, long lda, double* ws, int mode, double* Yout, long ldy,
                     double* Wout, long ldw, double* R, long ldr, double* Aband, long ldband,
                     cudaStream_t st) {
   TsqrPlan plan = make_plan(m);
   if (plan.nlev >= kMaxLevels) return EVD_ERR_INVALID_ARG;
   EVD_TRY(finish_attr());
-  EVD_TRY(launch_pdl(tsqr_up_kernel, plan.T[0], kThreads, 0, st, plan, A, lda, ws, R,
-                     ldr));
   int nodes = 0;
   for (int l = 0; l < plan.nlev; ++l) nodes += plan.T[l];
+  EVD_TRY(launch_pdl(tsqr_up_kernel, nodes, kThreads, sizeof(UpSmem), st, plan, A, lda, ws, R,
+                     ldr));
   EVD_TRY(launch_pdl(tsqr_q_kernel, nodes, kThreads, sizeof(QSmem), st, plan, A, lda,
                      ws));
   EVD_TRY(launch_pdl(tsqr_finish_kernel, plan.T[0], kThreads, sizeof(FinishSmem), st,
