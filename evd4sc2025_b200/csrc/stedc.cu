@@ -1000,14 +1000,10 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
   EVD_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
   absmax_kernel<<<1, 1024, 0, st>>>(n, d, e, scal);
   EVD_LAUNCHED();
-  {
-    // A NaN or Inf entry would break the merge ordering (ranks of NaN keys
-    // collide); reject it before any merge runs.
-    double h = 0.0;
-    EVD_CUDA_TRY(cudaMemcpyAsync(&h, scal, sizeof(double), cudaMemcpyDeviceToHost, st));
-    EVD_CUDA_TRY(cudaStreamSynchronize(st));
-    if (!isfinite(h)) return EVD_ERR_INVALID_ARG;
-  }
+  // A NaN or Inf entry would break the merge ordering (ranks of NaN keys
+  // collide): the norm is read with the first level's sizes, before any column
+  // moves, and such input is rejected there.
+  double hnorm = 0.0;
   double* dw = work + P.o_d;
   double* ew = work + P.o_e;
   double* Zw = work + P.o_Z;
@@ -1063,7 +1059,10 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
     hdesc.resize(8 * a.nm);
     EVD_CUDA_TRY(cudaMemcpyAsync(hdesc.data(), a.desc, sizeof(int) * 8 * a.nm,
                                  cudaMemcpyDeviceToHost, st));
+    if (lev == 1)
+      EVD_CUDA_TRY(cudaMemcpyAsync(&hnorm, scal, sizeof(double), cudaMemcpyDeviceToHost, st));
     EVD_CUDA_TRY(cudaStreamSynchronize(st));
+    if (!isfinite(hnorm)) return EVD_ERR_INVALID_ARG;
     int Kmax = 0, K12 = 0, K23 = 0, nrmax = 0;
     for (int m = 0; m < a.nm; ++m) {
       const int* dd = &hdesc[8 * m];
@@ -1138,6 +1137,11 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
     EVD_TRY(launch_pdl(merge_copy_deflated_kernel, gC, 256, 0, st, a));
     EVD_TRY(launch_pdl(merge_finalize_rank_kernel, gN, 256, 0, st, a));
     EVD_TRY(launch_pdl(merge_scatter_kernel, gC, 256, 0, st, a));
+  }
+  if (P.L == 0) {
+    EVD_CUDA_TRY(cudaMemcpyAsync(&hnorm, scal, sizeof(double), cudaMemcpyDeviceToHost, st));
+    EVD_CUDA_TRY(cudaStreamSynchronize(st));
+    if (!isfinite(hnorm)) return EVD_ERR_INVALID_ARG;
   }
   dim3 gf(ceil_div_i(n, 256), (unsigned)std::min<long>(n, 65535));
   if (out_after) EVD_CUDA_TRY(cudaStreamWaitEvent(st, out_after, 0));
