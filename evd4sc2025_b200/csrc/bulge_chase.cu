@@ -88,36 +88,13 @@ __device__ __forceinline__ void tile_store(double* sub, const double* t, long c0
   for (int i = threadIdx.x; i < n2; i += kChaseThreads) __stcg(dst + i, src[i]);
 }
 
-// Reductions on the tensor pipe.  Inside a chase step the warp shuffles queue
-// behind the shared-memory traffic of the tile copies (a 5-level shuffle sum
-// took about 2400 cycles there, 190 alone); the DMMA unit is otherwise idle.
-// mma.m8n8k4.f64 fragments: lane l holds A[l/4][l%4], B[l%4][l/4] and
-// D[l/4][2(l%4)], D[l/4][2(l%4)+1].
-__device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
-  asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%5};\n"
-      : "=d"(d0), "=d"(d1)
-      : "d"(a), "d"(b), "d"(0.0), "d"(0.0));
-}
-
+// Quad and warp sums run on the tensor pipe: inside a chase step the warp
+// shuffles queue behind the shared-memory traffic of the tile copies (a 5-level
+// shuffle sum took about 2400 cycles there, 190 alone).
 // Sum over each quad of lanes (4i .. 4i+3): A = values, B = ones.
 __device__ __forceinline__ double quad_sum_tc(double v) {
   double d0, d1;
   dmma884(d0, d1, v, 1.0);
-  return d0;
-}
-
-// Sum over the warp, returned to every lane: quad sums s_i (A = values,
-// B = ones); then B2[0][j] = s_j gives D = s_j per column, so lane l holds
-// s_{2(l%4)} and s_{2(l%4)+1}; their sum u_{l%4} as A3[i][k] = u_k against
-// ones adds the four u_k.
-__device__ __forceinline__ double warp_sum_tc(double v) {
-  const int lane = threadIdx.x & 31;
-  double d0, d1;
-  dmma884(d0, d1, v, 1.0);
-  dmma884(d0, d1, 1.0, (lane & 3) == 0 ? d0 : 0.0);
-  const double u = d0 + d1;
-  dmma884(d0, d1, u, 1.0);
   return d0;
 }
 

@@ -161,6 +161,22 @@ __device__ __forceinline__ bool wait_msg(const Word2* m, unsigned flag, int* err
   }
 }
 
+// Both messages of a task in one loop (a wait costs 200 cycles even when the
+// message is there): entry l of the reflector, and of the column entry l, or
+// its diagonal only.
+template <bool DIAG>
+__device__ __forceinline__ bool wait_both(const Word2* u, unsigned fu, const Word2* c, unsigned fc,
+                                          int* err, Word2& mu, Word2& mc) {
+  const int lane = threadIdx.x & 31;
+  Patience pat;
+  for (unsigned it = 1;; ++it) {
+    mu = ld_sh(u + lane);
+    mc = ld_sh(DIAG ? c + kPB : c + lane);
+    if (__all_sync(0xffffffffu, has(mu, fu) && has(mc, fc))) return true;
+    if ((it & 255u) == 0 && pat.over(err)) return false;
+  }
+}
+
 struct PipeArgs {
   int n, s0, s1;  // sweeps [s0, s1), s1 <= n - 2
   double* sub;
@@ -239,17 +255,18 @@ __device__ __forceinline__ void run_n(const PipeArgs& a, SlotSmem& sm, const Des
     const int par = s & 1;
     const unsigned flag = (unsigned)(s + 1);
     Word2 m, dm;
-    if (s > a.s0) {
-      N[kPB - 1] = 0.0;
-      if (r + 31 <= n - 1) {
-        if (!wait_msg<true, false>(sm.in.c[par ^ 1], (unsigned)s, a.err, m, dm)) return;
-        N[kPB - 1] = unpack(m);
-      }
-    }
     double u = 0.0;
-    if (r <= n - 2) {
-      if (!wait_msg<true, false>(sm.in.u[par], flag, a.err, m, dm)) return;
+    if (s > a.s0 && r + 31 <= n - 1) {  // then r <= n - 2: a reflector comes too
+      if (!wait_both<false>(sm.in.u[par], flag, sm.in.c[par ^ 1], (unsigned)s, a.err, m, dm))
+        return;
       u = unpack(m);
+      N[kPB - 1] = unpack(dm);
+    } else {
+      if (s > a.s0) N[kPB - 1] = 0.0;
+      if (r <= n - 2) {
+        if (!wait_msg<true, false>(sm.in.u[par], flag, a.err, m, dm)) return;
+        u = unpack(m);
+      }
     }
     sm.un[li] = u;
     __syncwarp();
@@ -265,7 +282,7 @@ __device__ __forceinline__ void run_n(const PipeArgs& a, SlotSmem& sm, const Des
     const double w = (w0 + w1) + (w2 + w3);
     const double x = fma(-w, sm.un[0], N[0]);
     const double x0 = __shfl_sync(0xffffffffu, x, rho);
-    const double nrm2 = warp_sum(x * x);
+    const double nrm2 = warp_sum_tc(x * x);
     double up = 0.0, up0 = 0.0, beta = x0;
     if (next_real && nrm2 > 0.0) up = house(x, lane == rho, x0, nrm2, up0, beta);
     if (next_real) {
@@ -372,13 +389,14 @@ __device__ __forceinline__ void run_s(const PipeArgs& a, SlotSmem& sm, const Des
       }
       S[kPB - 2] = (li == 31) ? row[kPB - 2] : S[kPB - 2];
       S[kPB - 1] = (li == 31) ? 0.0 : row[li];
-      if (r + 31 <= n - 1) {
-        if (!wait_msg<true, true>(sm.in.c[par ^ 1], (unsigned)s, a.err, m, dm)) return;
-        if (li == 31) S[kPB - 1] = unpack(dm);
-      }
     }
     double u = 0.0;
-    if (r <= n - 2) {
+    if (s > a.s0 && r + 31 <= n - 1) {
+      if (!wait_both<true>(sm.in.u[par], flag, sm.in.c[par ^ 1], (unsigned)s, a.err, m, dm))
+        return;
+      u = unpack(m);
+      if (li == 31) S[kPB - 1] = unpack(dm);
+    } else if (r <= n - 2) {
       if (!wait_msg<true, false>(sm.in.u[par], flag, a.err, m, dm)) return;
       u = unpack(m);
     }
@@ -394,7 +412,7 @@ __device__ __forceinline__ void run_s(const PipeArgs& a, SlotSmem& sm, const Des
       y3 = fma(S[j + 3], ub.y, y3);
     }
     const double y = (y0 + y1) + (y2 + y3);
-    const double ht = 0.5 * warp_sum(u * y);
+    const double ht = 0.5 * warp_sum_tc(u * y);
     const double v = fma(-ht, u, y);
     sm.v[li] = v;
     __syncwarp();
@@ -433,7 +451,7 @@ __device__ void run_head(const PipeArgs& a, SlotSmem* slots, const Word2* headbo
       x = unpack(mine);
       d = unpack(dm);
     }
-    const double nrm2 = warp_sum(x * x);
+    const double nrm2 = warp_sum_tc(x * x);
     const double x0 = __shfl_sync(0xffffffffu, x, first);
     double u = 0.0, u0 = 0.0, beta = x0;
     if (nrm2 > 0.0) u = house(x, lane == first, x0, nrm2, u0, beta);
@@ -589,8 +607,10 @@ bool chase_pipelined(long n) {
 // a relay warp), which costs 0.3 us more per message; with 7 slots per CTA
 // (96 registers, the rows spill) where 4 would need more CTAs than SMs.
 // Measured on B200, ms per chase (chase_kernel -> this kernel) and us per sweep:
-//   n = 128: 0.83 -> 0.22 (1.7), 1024: 8.7 -> 1.5 (1.5), 2048: 18.0 -> 3.0 (1.5),
-//   4096: 36.5 -> 8.7 (2.1), 16384: 182 -> 35.3 (2.2), 20000: 55 (2.8).
+//   n = 128: 0.83 -> 0.22 (1.7), 1024: 8.7 -> 1.43 (1.4), 2048: 18.0 -> 2.8 (1.4),
+//   4096: 36.5 -> 8.5 (2.1), 16384: 182 -> 34.5 (2.1), 20000: 52 (2.6).
+// Inside a cluster the N warp is busy all the time (2750 of 2900 cycles, 600 of
+// them the reduce-scatter of z); above, the messages through L2 are the rest.
 int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* msg, long s0,
                       long s1, cudaStream_t st, bool* used) {
   *used = true;
