@@ -526,8 +526,10 @@ __global__ void __launch_bounds__(SL* kSlotThreads + 32 * kExtraWarps, 1)
   if (cluster && gridDim.x > 1) cg::this_cluster().sync();
 }
 
+// A launch that the device cannot hold at once (fewer SMs than it reports, no
+// such cluster) is refused by the runtime: *used turns false.
 template <int SL>
-int launch(const PipeArgs& a, int ctas, bool coop, cudaStream_t st) {
+int launch(const PipeArgs& a, int ctas, bool coop, cudaStream_t st, bool* used) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(SL * kSlotThreads + 32 * kExtraWarps);
@@ -545,7 +547,14 @@ int launch(const PipeArgs& a, int ctas, bool coop, cudaStream_t st) {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
   }
-  EVD_CUDA_TRY(cudaLaunchKernelEx(&cfg, chase_pipe_kernel<SL>, a));
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, chase_pipe_kernel<SL>, a);
+  if (rc == cudaErrorCooperativeLaunchTooLarge || rc == cudaErrorInvalidClusterSize ||
+      rc == cudaErrorInvalidConfiguration || rc == cudaErrorLaunchOutOfResources) {
+    (void)cudaGetLastError();
+    *used = false;
+    return EVD_SUCCESS;
+  }
+  EVD_CUDA_TRY(rc);
   EVD_LAUNCHED();
   return EVD_SUCCESS;
 }
@@ -620,13 +629,13 @@ int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* m
   if (need <= 8 || (need <= 16 && cluster16_fits())) {
     int c = 1;
     while (c < need) c *= 2;
-    return launch<kSlA>(a, c, false, st);
+    return launch<kSlA>(a, c, false, st, used);
   }
   a.bnd = reinterpret_cast<Boundary*>(((uintptr_t)msg + 15) & ~(uintptr_t)15);
   const int most = std::min(device_sm_count(), kMaxPipeCtas);
-  if (need <= most) return launch<kSlA>(a, need, true, st);
+  if (need <= most) return launch<kSlA>(a, need, true, st, used);
   const int needb = (slots + kSlB - 1) / kSlB;
-  if (needb <= most) return launch<kSlB>(a, needb, true, st);
+  if (needb <= most) return launch<kSlB>(a, needb, true, st, used);
   *used = false;
   return EVD_SUCCESS;
 }
