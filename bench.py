@@ -11,7 +11,7 @@ orthogonality <= 1e-13 (checked on the result of the timed solves).
 
 * value:   device time per EVD of the MIXED form (evd_syevd_mixed: the big
            contractions as emulated FP64 products on the int8 tensor cores,
-           the stage-2 reflectors accumulated in two chains beside the chase,
+           the stage-2 reflectors accumulated in two chains after the chase,
            Q1 formed and the divide and conquer run beside them), A already
            resident in HBM (CUDA events on the
            solver stream, W warm-up steps, K timed steps, max over ranks);
@@ -394,11 +394,11 @@ def run_ours(args) -> int:
     # the mixed form's critical path) and the int8 tensor-core GEMM ----
     bc_ms = stages_p.get("bc_back", float("nan"))
     achieved = 2.0 * n ** 3 / (bc_ms * 1e-3) / 1e12
-    # DRAM bytes of one q2_mma_kernel launch: 34.33e9 measured by ncu at n=8192
+    # DRAM bytes of one q2_mma8_kernel launch: 33.95e9 measured by ncu at n=8192
     # (dram__bytes_read.sum + dram__bytes_write.sum), growing as n^3 (each of
     # the n/128 strips streams the rows of X below it once)
-    traffic = 34.33e9 * (n / 8192.0) ** 3
-    roofline = {"kernel": "q2_mma_kernel (stage-2 back transformation on DMMA)",
+    traffic = 33.95e9 * (n / 8192.0) ** 3
+    roofline = {"kernel": "q2_mma8_kernel (stage-2 back transformation on DMMA)",
                 "bound": "fp64", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp64_peak, "traffic": traffic,
                 "traffic_source": "ncu capture at n=8192 scaled by (n/8192)^3",

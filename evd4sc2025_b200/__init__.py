@@ -486,8 +486,7 @@ def syevd_s(A: torch.Tensor, b: int = 32, nb: int = 1024, work: torch.Tensor | N
 def mixed_last_timings() -> dict:
     """Stage times (ms) of the last timed :func:`syevd_mixed` on this thread.
     q1_formation and stage2_chains (the stage-2 reflectors accumulated from the
-    identity, one chase range behind the chase) run on side streams beside the
-    chase and the divide and conquer; final_products (from the end of the
+    identity after the chase) run on side streams beside the divide and conquer; final_products (from the end of the
     divide and conquer to X) includes waiting for them."""
     out = (C.c_double * 8)()
     lib().evd_syevd_mixed_last_timings(out)

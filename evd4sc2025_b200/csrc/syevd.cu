@@ -419,7 +419,7 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
     EVD_CUDA_TRY(cudaStreamWaitEvent(sc, ev[2], 0));
     EVD_TRY(set_identity(n, n, X, ldX, sc));
   }
-  // ---- main: the chase, one launch per sweep range ----
+  // ---- main: the chase ----
   {
     NvtxRange r("evd_b200 bulge chasing");
     EVD_CUDA_TRY(cudaMemsetAsync(U, 0, sizeof(double) * n * n, st));
@@ -430,9 +430,9 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
     EVD_TRY(chase_tridiag(n, sub, 2 * b, d, e, st));
   }
   EVD_CUDA_TRY(cudaEventRecord(ev[4], st));
-  // ---- the chains, range by range behind the chase ----
+  // ---- the chains (a chase in ranges: range by range behind it) ----
   {
-    NvtxRange r("evd_b200 stage-2 reflectors beside the chase (side streams)");
+    NvtxRange r("evd_b200 stage-2 reflectors (side streams)");
     // The pipelined kernel's counters into Z and R (free after stage 1).  Where
     // the 64-column CTAs of the plain kernel fill the SMs it is the better
     // neighbour of the divide and conquer and the Q1 formation: n = 16384 833 ms

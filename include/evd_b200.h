@@ -332,7 +332,7 @@ double evd_syevd_last_refine_ms(void);
  * stage-2 chains (from their start to the end of the later one), the final
  * products (from the end of the divide and conquer to X), refinement, total.
  * The Q1 formation and the stage-2 chains run on side streams beside the
- * chase and the divide and conquer. */
+ * divide and conquer. */
 void evd_syevd_mixed_last_timings(double out_ms[8]);
 
 /* ---- FP32 solve ---------------------------------------------------------- */
