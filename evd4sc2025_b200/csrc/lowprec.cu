@@ -656,8 +656,14 @@ int tc_syr2k_run(long n, long k, float alpha, const TI* A, long lda, const TI* B
 
 }  // namespace
 
-// `count` ints from the pool, freed with cudaFreeAsync; nullptr when there are none.
+// `count` ints from the pool, freed with cudaFreeAsync; nullptr when there are
+// none, and in a stream capture (a captured call allocates nothing).
 int* pool_ints(long count, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
   cudaMemPool_t pool = lp_pool();
   int* p = nullptr;
   if (!pool || cudaMallocFromPoolAsync((void**)&p, sizeof(int) * (size_t)count, pool, st) !=
