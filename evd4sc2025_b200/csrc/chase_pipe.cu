@@ -60,6 +60,20 @@ struct __align__(16) Word2 {
   u64 lo, hi;  // (flag << 32) | half of the double
 };
 
+// Slot k has a task in sweep s while its window's first row r = s + 1 + 32 k is
+// a row of the matrix.  Every task waits for the reflector message of its
+// sweep, also the last one (r = n - 1), which has nothing to reflect and gets a
+// zero: that message is what orders a slot's two warps and its neighbours.
+// u(s) to slot k is sent by slot k-1 after it has read c(s-1), which S(k) sent
+// after it had read u(s-1) and the row of sweep s-2; so whoever holds u(s) may
+// write over everything that was two sweeps old.
+__host__ __device__ constexpr int last_sweep(int n, int s1, int k) {
+  return s1 - 1 < n - 2 - kPB * k ? s1 - 1 : n - 2 - kPB * k;
+}
+__host__ __device__ constexpr bool has_next_slot(int n, int r) { return r + kPB <= n - 1; }
+// its column r + 31 exists: a column message of the sweep before comes too
+__host__ __device__ constexpr bool takes_column(int n, int r) { return r + kPB - 1 <= n - 1; }
+
 // A slot's inbox: reflector and column messages, two sweeps deep (a sender can
 // be at most one sweep ahead of the last message its receiver has read).
 // Entry 32 of a column is its diagonal element; entry (c mod 32) of column c
@@ -247,27 +261,23 @@ __device__ __forceinline__ void run_n(const PipeArgs& a, SlotSmem& sm, const Des
     for (int j = 0; j < kPB; ++j)
       N[j] = (r + kPB + li < n) ? a.sub[(long)(r + j) * kPOff + (kPB + li - j)] : 0.0;
   }
-  const int last = min(a.s1 - 1, n - 2 - kPB * k);  // the window starts at row <= n - 1
+  const int last = last_sweep(n, a.s1, k);
   for (int s = a.s0; s <= last; ++s, ++r) {
     const int rho = (s + 1) & 31;  // lane of N's first row
     const int li = (lane - rho) & 31;
-    const bool next_real = r + kPB <= n - 2;
+    const bool next_real = r + kPB <= n - 2;  // a reflector of two rows or more
     const int par = s & 1;
     const unsigned flag = (unsigned)(s + 1);
     Word2 m, dm;
-    double u = 0.0;
-    if (s > a.s0 && r + 31 <= n - 1) {  // then r <= n - 2: a reflector comes too
+    if (s > a.s0 && takes_column(n, r)) {
       if (!wait_both<false>(sm.in.u[par], flag, sm.in.c[par ^ 1], (unsigned)s, a.err, m, dm))
         return;
-      u = unpack(m);
       N[kPB - 1] = unpack(dm);
     } else {
       if (s > a.s0) N[kPB - 1] = 0.0;
-      if (r <= n - 2) {
-        if (!wait_msg<true, false>(sm.in.u[par], flag, a.err, m, dm)) return;
-        u = unpack(m);
-      }
+      if (!wait_msg<true, false>(sm.in.u[par], flag, a.err, m, dm)) return;
     }
+    const double u = unpack(m);
     sm.un[li] = u;
     __syncwarp();
     double w0 = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0;
@@ -285,10 +295,10 @@ __device__ __forceinline__ void run_n(const PipeArgs& a, SlotSmem& sm, const Des
     const double nrm2 = warp_sum_tc(x * x);
     double up = 0.0, up0 = 0.0, beta = x0;
     if (next_real && nrm2 > 0.0) up = house(x, lane == rho, x0, nrm2, up0, beta);
-    if (next_real) {
+    if (has_next_slot(n, r)) {
       du.put(par * kPB + lane, up, flag);
       const int row = r + kPB + li;
-      if (a.U != nullptr && row < n) a.U[row + (long)s * a.ldU] = up;
+      if (next_real && a.U != nullptr && row < n) a.U[row + (long)s * a.ldU] = up;
     }
     if (s < a.s1 - 1 && lane == rho) dc.put(par * (kPB + 1) + rho, beta, flag);
     // ---- off the critical cycle: N <- N - w u^T, z = N^T u', N <- N - u' z^T,
@@ -334,7 +344,7 @@ __device__ __forceinline__ void run_n(const PipeArgs& a, SlotSmem& sm, const Des
 #pragma unroll
         for (int j = 1; j < kPB; ++j) p[(long)j * (kPOff - 1)] = N[j - 1];
       }
-    } else {
+    } else if (s < last) {
       // the first row leaves for S; its lane takes the new last row (empty but
       // for the column that the next message brings)
       if (lane == rho) {
@@ -366,7 +376,7 @@ __device__ __forceinline__ void run_s(const PipeArgs& a, SlotSmem& sm, const Des
       S[j] = (r + hi < n) ? a.sub[(long)(r + lo) * kPOff + (hi - lo)] : 0.0;
     }
   }
-  const int last = min(a.s1 - 1, n - 2 - kPB * k);
+  const int last = last_sweep(n, a.s1, k);
   for (int s = a.s0; s <= last; ++s, ++r) {
     const int rho = (s + 1) & 31;
     const int li = (lane - rho) & 31;
@@ -390,16 +400,14 @@ __device__ __forceinline__ void run_s(const PipeArgs& a, SlotSmem& sm, const Des
       S[kPB - 2] = (li == 31) ? row[kPB - 2] : S[kPB - 2];
       S[kPB - 1] = (li == 31) ? 0.0 : row[li];
     }
-    double u = 0.0;
-    if (s > a.s0 && r + 31 <= n - 1) {
+    if (s > a.s0 && takes_column(n, r)) {
       if (!wait_both<true>(sm.in.u[par], flag, sm.in.c[par ^ 1], (unsigned)s, a.err, m, dm))
         return;
-      u = unpack(m);
       if (li == 31) S[kPB - 1] = unpack(dm);
-    } else if (r <= n - 2) {
+    } else {
       if (!wait_msg<true, false>(sm.in.u[par], flag, a.err, m, dm)) return;
-      u = unpack(m);
     }
+    const double u = unpack(m);
     sm.us[li] = u;
     __syncwarp();
     double y0 = 0.0, y1 = 0.0, y2 = 0.0, y3 = 0.0;
@@ -466,7 +474,7 @@ __device__ void run_head(const PipeArgs& a, SlotSmem* slots, const Word2* headbo
 // Cooperative launch: messages of the neighbour CTAs, global -> shared memory.
 __device__ void run_relay_u(const PipeArgs& a, SlotSmem* slots, int k) {
   const int lane = threadIdx.x & 31;
-  const int last = min(a.s1 - 1, a.n - 3 - kPB * k);  // slot k works on a real sweep
+  const int last = last_sweep(a.n, a.s1, k);
   const Boundary* b = a.bnd + blockIdx.x - 1;
   for (int s = a.s0; s <= last; ++s) {
     Word2 mine, dm;
@@ -477,10 +485,9 @@ __device__ void run_relay_u(const PipeArgs& a, SlotSmem* slots, int k) {
 template <int SL>
 __device__ void run_relay_c(const PipeArgs& a, SlotSmem* slots, int k) {
   const int lane = threadIdx.x & 31;
-  // column r + 31 <= n - 1 with r = s + 1 + 32 k
-  const int last = min(a.s1 - 1, a.n - 33 - kPB * k);
+  const int last = last_sweep(a.n, a.s1, k);
   const Boundary* b = a.bnd + blockIdx.x;
-  for (int s = a.s0 + 1; s <= last; ++s) {
+  for (int s = a.s0 + 1; s <= last && takes_column(a.n, s + 1 + kPB * k); ++s) {
     Word2 mine, dm;
     const int q = (s & 1) ^ 1;
     if (!wait_msg<false, true>(b->c[q], (unsigned)s, a.err, mine, dm)) return;
@@ -641,3 +648,15 @@ int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* m
 }
 
 }  // namespace evd
+
+// The flow of messages as the kernel has it, for the host's check of the order
+// it imposes: out = {last sweep of slot k, its task in sweep s waits for a
+// reflector, waits for a column, sends a reflector, hands a row from N to S}.
+extern "C" void evd_test_chase_flow(int n, int s0, int s1, int k, int s, int out[5]) {
+  const int r = s + 1 + evd::kPB * k;
+  out[0] = evd::last_sweep(n, s1, k);
+  out[1] = 1;
+  out[2] = s > s0 && evd::takes_column(n, r);
+  out[3] = evd::has_next_slot(n, r);
+  out[4] = s < s1 - 1 && s < out[0];
+}
