@@ -157,22 +157,30 @@ struct Patience {
   }
 };
 
+// The one loop that every wait of a warp runs in: all lanes leave it in the same
+// turn, as the full-mask shuffle of over() needs.
+template <typename Ready>
+__device__ __forceinline__ bool wait_warp(int* err, Ready ready) {
+  Patience pat;
+  for (unsigned it = 1; !__all_sync(0xffffffffu, ready()); ++it)
+    if ((it & 255u) == 0 && pat.over(err)) return false;
+  return true;
+}
+
 // Warp-wide wait for a message of 32 entries (and a 33rd): lane l polls entry l.
 template <bool SHARED, bool DIAG>
 __device__ __forceinline__ bool wait_msg(const Word2* m, unsigned flag, int* err, Word2& mine,
                                          Word2& diag) {
   const int lane = threadIdx.x & 31;
-  Patience pat;
-  for (unsigned it = 1;; ++it) {
+  return wait_warp(err, [&] {
     mine = SHARED ? ld_sh(m + lane) : ld_any(m + lane);
     bool good = has(mine, flag);
     if (DIAG) {
       diag = SHARED ? ld_sh(m + kPB) : ld_any(m + kPB);
       good = good && has(diag, flag);
     }
-    if (__all_sync(0xffffffffu, good)) return true;
-    if ((it & 255u) == 0 && pat.over(err)) return false;
-  }
+    return good;
+  });
 }
 
 // Both messages of a task in one loop (a wait costs 200 cycles even when the
@@ -182,13 +190,11 @@ template <bool DIAG>
 __device__ __forceinline__ bool wait_both(const Word2* u, unsigned fu, const Word2* c, unsigned fc,
                                           int* err, Word2& mu, Word2& mc) {
   const int lane = threadIdx.x & 31;
-  Patience pat;
-  for (unsigned it = 1;; ++it) {
+  return wait_warp(err, [&] {
     mu = ld_sh(u + lane);
     mc = ld_sh(DIAG ? c + kPB : c + lane);
-    if (__all_sync(0xffffffffu, has(mu, fu) && has(mc, fc))) return true;
-    if ((it & 255u) == 0 && pat.over(err)) return false;
-  }
+    return has(mu, fu) && has(mc, fc);
+  });
 }
 
 struct PipeArgs {
@@ -385,10 +391,7 @@ __device__ __forceinline__ void run_s(const PipeArgs& a, SlotSmem& sm, const Des
     Word2 m, dm;
     if (s > a.s0) {
       // the row that left N in the last sweep is row and column r + 31 now
-      Patience pat;
-      for (unsigned it = 1; *(volatile int*)&sm.row_flag[par ^ 1] != s; ++it)
-        if ((it & 255u) == 0 && pat.over(a.err)) return;
-      __syncwarp();
+      if (!wait_warp(a.err, [&] { return *(volatile int*)&sm.row_flag[par ^ 1] == s; })) return;
       __threadfence_block();
       const double* row = sm.row[par ^ 1];
 #pragma unroll

@@ -10,6 +10,8 @@ builds that relation with vector clocks from the kernel's own conditions
 (evd_test_chase_flow) and also sees that every wait ends.
 """
 import ctypes as C
+import pathlib
+import re
 
 import pytest
 
@@ -126,3 +128,14 @@ def test_the_check_sees_an_unordered_last_task():
     bad, stuck = check(programs(former_flow, 131, 0, 129, 4, False))
     assert not stuck
     assert {b[2][0] for b in bad} == {"row", "c"}  # both places: the row and S's column
+
+
+def test_every_bounded_wait_leaves_its_loop_as_a_whole_warp():
+    """Patience::over shuffles with the full mask, so its loop may only be left
+    by a vote of the warp: one loop, and every wait goes through it."""
+    src = (pathlib.Path(__file__).resolve().parents[1] / "evd4sc2025_b200" / "csrc"
+           / "chase_pipe.cu").read_text()
+    calls = [m.start() for m in re.finditer(r"\.over\(", src)]
+    assert len(calls) == 1
+    loop = src[src.rindex("for (", 0, calls[0]):calls[0]]
+    assert "!__all_sync(0xffffffffu, ready())" in loop
