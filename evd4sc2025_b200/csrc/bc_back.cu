@@ -42,11 +42,14 @@
 // the DMMA pipe (parallelogram padding 40/32, plus the T product), plus the
 // Gram products.  Rows >= n are never read or written (the reference needs
 // 346 zero rows of padding).
+#include <vector>
+
 #include "common.cuh"
 
 namespace evd {
 
 int* pool_ints(long count, cudaStream_t st);
+int read_device_error(const int* err_word, cudaStream_t st);
 
 namespace {
 
@@ -590,16 +593,20 @@ __device__ __forceinline__ void store_tile8(const double (&v)[2], double* cg, bo
 // CTAs take their work from a ticket, strip by strip, and wait only for a
 // strip that an earlier ticket owns, so some CTA can always go on.  prog[] holds
 // the blocks that each (strip, column block) has finished (its count + 1 at the
-// end), ticket and counters start at zero.  A wait that outlasts 4 s fills the
-// columns with NaN (nothing else could report it from here).
-// X passes between SMs, so PIPE reads it past L1.
+// end), ticket and counters start at zero.  When a wait runs out, the CTA
+// records it in the error word and fills all its columns with NaN: the
+// solvers report the word, evd_bc_back_apply (which does not synchronise) has
+// the NaN.  X passes between SMs, so PIPE reads it past L1.
 struct Q2Pipe {
   int* ticket;
   int* prog;
+  int* err;
+  unsigned long long limit;  // of a wait, ns
 };
 constexpr int kPubEvery = 4;  // blocks between two publications of progress
+constexpr unsigned long long kQ2LimitNs = 4000000000ull;
 
-__device__ __forceinline__ bool q2_wait(const int* flag, int need, int& seen) {
+__device__ __forceinline__ bool q2_wait(const int* flag, int need, int& seen, const Q2Pipe& pp) {
   if (seen >= need) return true;
   unsigned long long t0 = 0;
   for (unsigned it = 1;; ++it) {
@@ -609,7 +616,10 @@ __device__ __forceinline__ bool q2_wait(const int* flag, int need, int& seen) {
       unsigned long long t;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
       if (t0 == 0) t0 = t;
-      if (t - t0 > 4000000000ull) return false;
+      if (t - t0 > pp.limit) {
+        atomicCAS(pp.err, 0, kDevTimeoutStrips);
+        return false;
+      }
     }
   }
 }
@@ -675,7 +685,6 @@ __global__ void __launch_bounds__(NW * 32, 3)
     const int* dflag = dep ? pp.prog + (long)(si - 1) * ncb + cb_at : nullptr;
     int* mine = PIPE ? pp.prog + (long)si * ncb + cb_at : nullptr;
     int cnt_d = 0, seen = 0;
-    bool ok = true;
     if (dep) {
       const int nb_d = nblk + (FWD ? -kStrip / 8 : kStrip / 8);
       cnt_d = (RANGE ? min(nb_d, (rg.h1 + 7) / 8) : nb_d) - bbA;
@@ -688,19 +697,25 @@ __global__ void __launch_bounds__(NW * 32, 3)
       return (it >= cnt - 1 || k > cnt_d) ? cnt_d + 1 : k;
     };
 
-    if (PIPE && dep && threadIdx.x == 0) ok = q2_wait(dflag, need_of(-1), seen);
-    if (PIPE) {
-      ok = __syncthreads_and(ok) != 0;
-      if (!ok) {
-        for (int i = 0; i < n; ++i)
-          if (okg && t == 0) cg[i] = __longlong_as_double(0x7ff8000000000000ll);
+    // the barrier at the head of an iteration, which also gives every thread
+    // thread 0's verdict on the strip before
+    auto enter = [&](int it) {
+      if (!PIPE) {
         __syncthreads();
-        if (threadIdx.x == 0) st_release(mine, cnt + 1);
-        return;
+        return true;
       }
-    } else {
+      const bool ok = threadIdx.x != 0 || !dep || q2_wait(dflag, need_of(it), seen, pp);
+      return __syncthreads_and(ok) != 0;
+    };
+    auto give_up = [&] {
+      if (okg && t == 0)
+        for (int i = 0; i < n; ++i) cg[i] = __longlong_as_double(0x7ff8000000000000ll);
+      cp_wait<0>();
       __syncthreads();
-    }
+      if (threadIdx.x == 0) st_release(mine, cnt + 1);
+    };
+
+    if (!enter(-1)) return give_up();
     {
       const long base = R + 8L * bb_of(0) + 1;
 #pragma unroll
@@ -715,8 +730,7 @@ __global__ void __launch_bounds__(NW * 32, 3)
       const int bb = bb_of(it);
       const long base = R + 8L * bb + 1;
       cp_wait<0>();
-      if (PIPE && dep && ok && threadIdx.x == 0) ok = q2_wait(dflag, need_of(it), seen);
-      __syncthreads();
+      if (!enter(it)) return give_up();
       if (PIPE && threadIdx.x == 0 && it > 0 && it % kPubEvery == 0) st_release(mine, it);
       if (it + 1 < cnt) {
         stage_y(Ys + ((it + 1) & 1) * kYBuf, R, H, bb_of(it + 1));
@@ -752,8 +766,6 @@ __global__ void __launch_bounds__(NW * 32, 3)
       for (int i = 0; i < kTiles; ++i) store_tile8(x[i], cg, okg, base + 8 * i, t2, n);
     }
     if (PIPE) {
-      if (threadIdx.x == 0 && !ok)  // a wait ran out: visible in the result
-        for (int i = 0; i < n; ++i) cg[i] = __longlong_as_double(0x7ff8000000000000ll);
       __syncthreads();
       if (threadIdx.x == 0) {
         __threadfence();
@@ -763,7 +775,8 @@ __global__ void __launch_bounds__(NW * 32, 3)
   }
 }
 
-// Ints of the pipelined kernel's ticket and progress counters.
+// Ints of the pipelined kernel's ticket, error word (for callers without one of
+// their own) and progress counters.
 long q2_flag_ints(long n, long ncols) {
   return 4 + ((n - 2 + kStrip - 1) / kStrip) * ((ncols + 31) / 32);
 }
@@ -772,18 +785,19 @@ constexpr size_t kQ8Smem = (size_t)2 * (kYBuf + kVBuf) * sizeof(double);  // 4 C
 
 template <bool FWD, int NW, bool RANGE>
 int launch_q2_8(long n, long ncols, const double* U, long ldU, const double* Tg, double* X,
-                long ldX, Q2Range rg, int* flags, cudaStream_t st) {
+                long ldX, Q2Range rg, int* flags, int* err, cudaStream_t st) {
   const int ncb = ceil_div_i((int)ncols, NW * kQ8Cols);
   if (flags) {
     const int nstrips = (int)((n - 2 + kStrip - 1) / kStrip);
     EVD_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)q2_flag_ints(n, ncols), st));
     EVD_TRY(smem_attr_once((const void*)q2_mma8_kernel<FWD, NW, RANGE, true>, (int)kQ8Smem));
     q2_mma8_kernel<FWD, NW, RANGE, true><<<ncb * nstrips, NW * 32, kQ8Smem, st>>>(
-        (int)n, (int)ncols, U, ldU, Tg, X, ldX, rg, Q2Pipe{flags, flags + 4});
+        (int)n, (int)ncols, U, ldU, Tg, X, ldX, rg,
+        Q2Pipe{flags, flags + 4, err ? err : flags + 1, kQ2LimitNs});
   } else {
     EVD_TRY(smem_attr_once((const void*)q2_mma8_kernel<FWD, NW, RANGE, false>, (int)kQ8Smem));
     q2_mma8_kernel<FWD, NW, RANGE, false><<<ncb, NW * 32, kQ8Smem, st>>>(
-        (int)n, (int)ncols, U, ldU, Tg, X, ldX, rg, Q2Pipe{nullptr, nullptr});
+        (int)n, (int)ncols, U, ldU, Tg, X, ldX, rg, Q2Pipe{});
   }
   EVD_LAUNCHED();
   return EVD_SUCCESS;
@@ -811,14 +825,14 @@ int launch_q2(long n, long ncols, const double* U, long ldU, const double* Tg, d
 // without the range logic.
 template <bool FWD>
 int launch_q2_pre(long n, long ncols, const double* U, long ldU, const double* Tg, double* X,
-                  long ldX, Q2Range rg, int* flags, cudaStream_t st) {
+                  long ldX, Q2Range rg, int* flags, int* err, cudaStream_t st) {
   const bool whole = !rg.ident && rg.h0 == 0 && rg.h1 >= n - 2;
   if (n <= kStrip + 2) flags = nullptr;  // a single strip
   if (!flags && ncols >= 64L * device_sm_count())
     return whole ? launch_q2<FWD, true, false>(n, ncols, U, ldU, Tg, X, ldX, rg, st)
                  : launch_q2<FWD, true, true>(n, ncols, U, ldU, Tg, X, ldX, rg, st);
-  return whole ? launch_q2_8<FWD, 4, false>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, st)
-               : launch_q2_8<FWD, 4, true>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, st);
+  return whole ? launch_q2_8<FWD, 4, false>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, err, st)
+               : launch_q2_8<FWD, 4, true>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, err, st);
 }
 
 // -V fragments of the blocks of sweeps [h0, h1) in every strip.
@@ -844,7 +858,7 @@ long q2_tbuf_doubles(long n) {
 }
 
 int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, double* X,
-                   long ldX, double* tbuf, int* flags, long h0, long h1, long ident_k,
+                   long ldX, double* tbuf, int* flags, int* err, long h0, long h1, long ident_k,
                    cudaStream_t st) {
   const bool ident = ident_k >= 0;
   if (n < 0 || ncols < 0 || ldU < n || ldX < n) return EVD_ERR_INVALID_ARG;
@@ -861,18 +875,18 @@ int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, 
   if (tbuf) {
     if (forward) {
       EVD_TRY(launch_tbuild<true>(n, U, ldU, tbuf, h0, h1, st));
-      return launch_q2_pre<true>(n, ncols, U, ldU, tbuf, X, ldX, rg, flags, st);
+      return launch_q2_pre<true>(n, ncols, U, ldU, tbuf, X, ldX, rg, flags, err, st);
     }
     EVD_TRY(launch_tbuild<false>(n, U, ldU, tbuf, h0, h1, st));
-    return launch_q2_pre<false>(n, ncols, U, ldU, tbuf, X, ldX, rg, flags, st);
+    return launch_q2_pre<false>(n, ncols, U, ldU, tbuf, X, ldX, rg, flags, err, st);
   }
   return forward ? launch_q2<true, false, true>(n, ncols, U, ldU, nullptr, X, ldX, rg, st)
                  : launch_q2<false, false, true>(n, ncols, U, ldU, nullptr, X, ldX, rg, st);
 }
 
 int q2_apply(bool forward, long n, long ncols, const double* U, long ldU, double* X, long ldX,
-             double* tbuf, int* flags, cudaStream_t st) {
-  return q2_apply_range(forward, n, ncols, U, ldU, X, ldX, tbuf, flags, 0, n, -1, st);
+             double* tbuf, int* flags, int* err, cudaStream_t st) {
+  return q2_apply_range(forward, n, ncols, U, ldU, X, ldX, tbuf, flags, err, 0, n, -1, st);
 }
 
 // Ints of the optional `flags` scratch of q2_apply (0: of no use).
@@ -888,7 +902,7 @@ extern "C" long evd_bc_back_work_size(long n) { return evd::q2_tbuf_doubles(n < 
 extern "C" int evd_bc_back(double* Q, long ldQ, const double* U, long ldU, long n, int b,
                            cudaStream_t stream) {
   if (b != 32) return EVD_ERR_INVALID_ARG;
-  return evd::q2_apply(true, n, n, U, ldU, Q, ldQ, nullptr, nullptr, stream);
+  return evd::q2_apply(true, n, n, U, ldU, Q, ldQ, nullptr, nullptr, nullptr, stream);
 }
 
 extern "C" int evd_bc_back_apply(long n, long ncols, const double* U, long ldU, double* X,
@@ -900,7 +914,31 @@ extern "C" int evd_bc_back_apply(long n, long ncols, const double* U, long ldU, 
   int* flags = nullptr;
   const long nf = work ? evd::q2_flags(n, ncols) : 0;
   if (nf > 0 && ldU >= n && ldX >= n && U && X) flags = evd::pool_ints(nf, stream);
-  const int rc = evd::q2_apply(false, n, ncols, U, ldU, X, ldX, work, flags, stream);
+  const int rc = evd::q2_apply(false, n, ncols, U, ldU, X, ldX, work, flags, nullptr, stream);
   if (flags) EVD_CUDA_TRY(cudaFreeAsync(flags, stream));
   return rc;
+}
+
+// For the tests: the reverse application with the strip that is taken first left
+// out, its counters standing at `done` blocks, and waits of `limit` ns: every
+// later strip's wait runs out, at its first window or inside the strip.
+// flags: q2_flags(n, ncols) ints; returns the status that a solver would.
+extern "C" int evd_test_bc_back_timeout(long n, long ncols, const double* U, long ldU, double* X,
+                                        long ldX, double* work, int* flags, int done, long limit,
+                                        cudaStream_t stream) {
+  using namespace evd;
+  if (q2_flags(n, ncols) == 0 || limit > 1000000000) return EVD_ERR_INVALID_ARG;
+  const int ncb = ceil_div_i(ncols, 32), nstrips = (int)((n - 2 + kStrip - 1) / kStrip);
+  EVD_TRY(launch_tbuild<false>(n, U, ldU, work, 0, n, stream));
+  std::vector<int> h(q2_flags(n, ncols), 0);
+  h[0] = ncb;  // the tickets of the first strip are gone
+  for (int i = 0; i < ncb; ++i) h[4 + i] = done;
+  EVD_CUDA_TRY(cudaMemcpy(flags, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
+  const auto kern = q2_mma8_kernel<false, 4, false, true>;
+  EVD_TRY(smem_attr_once((const void*)kern, (int)kQ8Smem));
+  kern<<<ncb * (nstrips - 1), 128, kQ8Smem, stream>>>(
+      (int)n, (int)ncols, U, ldU, work, X, ldX, Q2Range{0, (int)n, 0, 0, 0},
+      Q2Pipe{flags, flags + 4, flags + 1, (unsigned long long)limit});
+  EVD_LAUNCHED();
+  return read_device_error(flags + 1, stream);
 }

@@ -395,7 +395,8 @@ int read_device_error(const int* err_word, cudaStream_t st) {
   int h = 0;
   EVD_CUDA_TRY(cudaMemcpyAsync(&h, err_word, sizeof(int), cudaMemcpyDeviceToHost, st));
   EVD_CUDA_TRY(cudaStreamSynchronize(st));
-  if (h == kDevTimeoutChase || h == kDevTimeoutTree) return EVD_ERR_TIMEOUT;
+  if (h == kDevTimeoutChase || h == kDevTimeoutTree || h == kDevTimeoutStrips)
+    return EVD_ERR_TIMEOUT;
   if (h == kDevNoConvergence) return EVD_ERR_NO_CONVERGENCE;
   if (h != 0) return EVD_ERR_INVALID_ARG;
   return EVD_SUCCESS;

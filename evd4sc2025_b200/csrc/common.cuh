@@ -52,6 +52,7 @@ enum DeviceError : int {
   kDevTimeoutTree = 2,
   kDevBadShape = 3,
   kDevNoConvergence = 4,
+  kDevTimeoutStrips = 5,
 };
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -43,10 +43,10 @@ int stedc(long n, double* d, double* e, double* Z, long ldz, double* work, long 
 long stedc_oz_bytes(long n, int nmod);
 long q2_tbuf_doubles(long n);
 int q2_apply(bool forward, long n, long ncols, const double* U, long ldU, double* X, long ldX,
-             double* tbuf, int* flags, cudaStream_t st);
+             double* tbuf, int* flags, int* err, cudaStream_t st);
 int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, double* X,
-                   long ldX, double* tbuf, int* flags, long h0, long h1, long ident_k,
-                   cudaStream_t st);
+                   long ldX, double* tbuf, int* flags, int* err, long h0, long h1,
+                   long ident_k, cudaStream_t st);
 long q2_flags(long n, long ncols);
 bool chase_pipelined(long n);
 int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, int* iwork,
@@ -256,7 +256,7 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
     double* tbuf = ((size_t)q2_tbuf_doubles(n) <= (size_t)n * n) ? OA : nullptr;
     // the pipelined kernel's counters into Z (n nb doubles, free after stage 1)
     int* flags = (q2_flags(n, n) > 0 && q2_flags(n, n) <= 2 * n * nb) ? (int*)Z : nullptr;
-    EVD_TRY(q2_apply(false, n, n, U, n, X, ldX, tbuf, flags, st));
+    EVD_TRY(q2_apply(false, n, n, U, n, X, ldX, tbuf, flags, ich + n + 32, st));
   }
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[4], st));
   {
@@ -279,7 +279,7 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
     g_timings[5] = ms;
     for (auto& x : ev) cudaEventDestroy(x);
   }
-  // chasing error word (bounded waits) is checked once at the end
+  // the error word of the bounded waits (chase, stage-2 strips), read once
   if (err_out) {
     *err_out = ich + n + 32;
     return EVD_SUCCESS;
@@ -443,11 +443,11 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
     int* fl[2] = {fits ? (int*)Z : nullptr, fits ? (int*)R : nullptr};
     for (int i = 0; i < nr; ++i) {
       EVD_CUDA_TRY(cudaStreamWaitEvent(sa, evr[i], 0));
-      EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, fl[0],
+      EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, fl[0], ich + n + 32,
                              bounds[i], split ? k : bounds[i + 1], 0, sa));
       if (split) {
         EVD_CUDA_TRY(cudaStreamWaitEvent(sc, evr[i], 0));
-        EVD_TRY(q2_apply_range(true, n, n, U, n, X, ldX, tbuf, fl[1], k,
+        EVD_TRY(q2_apply_range(true, n, n, U, n, X, ldX, tbuf, fl[1], ich + n + 32, k,
                                bounds[i + 1], k, sc));
       }
     }

@@ -193,7 +193,9 @@ int evd_bc_back(double* Q, long ldQ, const double* U, long ldU, long n, int b,
  * evd_bc_back_work_size(n) doubles, about 5 n^2/8) receives the compact-WY
  * factors V = Y T of the reflector groups, built once for all columns (the
  * kernel's progress counters, one int per 128 rows and 32 columns, come from a
- * stream-ordered pool of the library, none in a stream capture); with
+ * stream-ordered pool of the library, none in a stream capture; columns in
+ * which a wait between its strips runs out, after 4 s, come back filled with
+ * NaN, since the call does not synchronise); with
  * work == NULL the T factors are rebuilt inside the apply kernel (slower). */
 long evd_bc_back_work_size(long n);
 int evd_bc_back_apply(long n, long ncols, const double* U, long ldU, double* X, long ldX,

@@ -158,3 +158,31 @@ def test_check_orthogonality(cuda, evdlib):
     Qp[:, 0] *= 1.001
     v2 = evdlib.check_orthogonality(evdlib.to_cm(torch.from_numpy(Qp), device=cuda))
     assert abs(v2 - O.orthogonality(Qp)) <= 1e-6 * O.orthogonality(Qp)
+
+
+@pytest.mark.parametrize("done", [0, 17])
+@pytest.mark.parametrize("n,ncols", [(400, 33), (300, 70)])
+def test_a_strip_wait_that_runs_out_marks_every_column(cuda, evdlib, n, ncols, done):
+    """The strip taken first never runs: the next one's wait ends at its first
+    window (done = 0) or inside the strip (17 blocks are reported done)."""
+    import ctypes as C
+    g = torch.Generator(device=cuda).manual_seed(n)
+    sub = torch.zeros(n, 64, dtype=torch.float64, device=cuda)
+    for o in range(33):
+        sub[: n - o, o] = torch.randn(n - o, generator=g, dtype=torch.float64, device=cuda)
+    _, _, U = evdlib.bulge_chase(sub.t(), 32)
+    X = evdlib.to_cm(torch.randn(n, ncols, generator=g, dtype=torch.float64, device=cuda),
+                     device=cuda)
+    ref = evdlib.bc_back_apply(X.clone(memory_format=torch.preserve_format), U)
+    Y = X.clone(memory_format=torch.preserve_format)
+    work = torch.empty(evdlib.lib().evd_bc_back_work_size(n), dtype=torch.float64, device=cuda)
+    flags = torch.zeros(4 + 8 * ((ncols + 31) // 32), dtype=torch.int32, device=cuda)
+    torch.cuda.synchronize()
+    rc = evdlib.lib().evd_test_bc_back_timeout(
+        C.c_long(n), C.c_long(ncols), C.c_void_p(U.data_ptr()), C.c_long(n),
+        C.c_void_p(Y.data_ptr()), C.c_long(n), C.c_void_p(work.data_ptr()),
+        C.c_void_p(flags.data_ptr()), C.c_int(done), C.c_long(2000000), None)
+    assert rc == -3  # EVD_ERR_TIMEOUT
+    assert torch.isnan(Y).any(dim=0).all()
+    # and the device goes on as before
+    assert torch.equal(evdlib.bc_back_apply(X, U), ref)
