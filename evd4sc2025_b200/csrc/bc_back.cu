@@ -49,7 +49,6 @@
 namespace evd {
 
 int* pool_ints(long count, cudaStream_t st);
-int read_device_error(const int* err_word, cudaStream_t st);
 
 namespace {
 

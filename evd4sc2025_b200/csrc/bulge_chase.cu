@@ -308,9 +308,11 @@ __global__ void band_pack_kernel(int n, int b, const double* __restrict__ A, lon
 }
 
 __global__ void band_to_tridiag_kernel(int n, const double* __restrict__ sub, long ldSub,
-                                       double* __restrict__ d, double* __restrict__ e) {
+                                       double* __restrict__ d, double* __restrict__ e,
+                                       const int* before, int* err) {
   long j = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (j >= n) return;
+  if (j == 0 && before != nullptr && *before != 0) atomicCAS(err, 0, *before);
   d[j] = sub[j * ldSub];
   if (j < n - 1) e[j] = sub[1 + j * ldSub];
 }
@@ -367,11 +369,15 @@ int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long 
   return EVD_SUCCESS;
 }
 
-// d and e from the chased band (after the last part).
-int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, cudaStream_t st) {
+// d and e from the chased band (after the last part).  before: an error word of
+// the stages before the chase (or nullptr), which goes on into the chase's, so
+// that the solvers read one.
+int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, const int* before,
+                  int* iwork, cudaStream_t st) {
   if (n <= 0) return EVD_SUCCESS;
   if (!dSub || !d || (n > 1 && !e)) return EVD_ERR_INVALID_ARG;
-  band_to_tridiag_kernel<<<ceil_div_i(n, 256), 256, 0, st>>>((int)n, dSub, ldSub, d, e);
+  band_to_tridiag_kernel<<<ceil_div_i(n, 256), 256, 0, st>>>((int)n, dSub, ldSub, d, e, before,
+                                                         before ? iwork + n + 32 : nullptr);
   EVD_LAUNCHED();
   return EVD_SUCCESS;
 }
@@ -381,14 +387,14 @@ int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, 
 // The tile copies need ldSub == 2b exactly (contiguous band columns) and a
 // 16-byte aligned dSub.
 int bulge_chase_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU,
-                      double* d, double* e, int* iwork, cudaStream_t st) {
+                      double* d, double* e, int* iwork, const int* before, cudaStream_t st) {
   if (n < 0 || b != kBW || ldSub != 2 * b || (dU && n > 0 && ldU < n)) return EVD_ERR_INVALID_ARG;
   if (((uintptr_t)dSub & 15u) != 0) return EVD_ERR_INVALID_ARG;
   if (n > (1L << 30)) return EVD_ERR_INVALID_ARG;
   if (n == 0) return EVD_SUCCESS;
   if (!dSub || !d || !iwork || (n > 1 && !e)) return EVD_ERR_INVALID_ARG;  // dU may be NULL
   EVD_TRY(chase_part_async(n, b, dSub, ldSub, dU, ldU, iwork, 0, n - 2, 0, st));
-  return chase_tridiag(n, dSub, ldSub, d, e, st);
+  return chase_tridiag(n, dSub, ldSub, d, e, before, iwork, st);
 }
 
 int read_device_error(const int* err_word, cudaStream_t st) {
@@ -415,7 +421,7 @@ extern "C" long evd_bulge_chase_iwork_size(long n) {
 
 extern "C" int evd_bulge_chase(long n, long b, double* dSub, long ldSub, double* dU, long ldU,
                                double* d, double* e, int* iwork, cudaStream_t stream) {
-  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iwork, stream);
+  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iwork, nullptr, stream);
   if (rc != EVD_SUCCESS || n <= 2) return rc;
   return evd::read_device_error(iwork + n + 32, stream);
 }
@@ -481,7 +487,7 @@ extern "C" int evd_bulge_chase_noalloc(long n, long b, double* dSub, long ldSub,
   EVD_TRY(evd::chase_noalloc_scratch(&iw));
   // bulge_chase_async clears the flags, ticket and error word of the scratch
   // (cudaMemsetAsync) before every launch, so a call never sees stale state.
-  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iw, stream);
+  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iw, nullptr, stream);
   if (rc != EVD_SUCCESS || n <= 2) return rc;
   return evd::read_device_error(iw + n + 32, stream);
 }

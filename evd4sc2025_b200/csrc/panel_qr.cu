@@ -41,6 +41,7 @@ constexpr int kNB = 32;           // panel width (reference: N = 32)
 constexpr int kFan = kTile / kNB; // children per tree node (their R factors fill one tile)
 constexpr int kThreads = 256;
 constexpr int kMaxLevels = 16;
+constexpr int kErrWord = 1, kCounters = 2;  // places among the ints of the workspace
 
 struct TsqrPlan {
   int m;
@@ -52,6 +53,7 @@ struct TsqrPlan {
   long qtop_off;            // 32x32 copy of the top of leaf 0's Q, row-major
   long cnt_off;             // int counters start (in doubles, aligned)
   int ncnt;
+  unsigned long long limit; // of a wait, ns
   long total;               // doubles
 };
 
@@ -70,7 +72,9 @@ TsqrPlan make_plan(long m) {
     ++L;
   }
   p.nlev = L + 1;
-  p.ncnt = 1 + kNB / 8 * coff;  // the ticket, a counter per inner node and column group
+  // the ticket, the error word, a counter per inner node and column group
+  p.ncnt = kCounters + kNB / 8 * coff;
+  p.limit = 4000000000ull;
   // Arrival counters come first, at a fixed offset: a workspace sized (and
   // zeroed) for the largest panel then serves every smaller panel, whose
   // counters are a prefix of the same region (the kernels reset each counter
@@ -133,8 +137,10 @@ __device__ __forceinline__ void row_block(const double* A, const double* B, int 
 // follows from the norm.
 //
 // Progress: CTAs take nodes from a ticket, leaves first, and wait only for
-// children, which earlier tickets own.  A wait that outlasts 4 s fills the
-// node's R with NaN, which the tridiagonal solver rejects.
+// children, which earlier tickets own.  When a wait runs out (4 s), the node
+// fills its R with NaN and sets the workspace's error word, which the solvers
+// report; the nodes and panels that follow wait no more (their counters may
+// hold late arrivals) and have NaN too.
 constexpr int kGrp = 8, kGroups = kNB / kGrp;
 constexpr int kWLd = kGrp + 4;  // row stride of 8-wide matrices (conflict-free fragments)
 
@@ -168,11 +174,12 @@ __global__ void __launch_bounds__(kThreads, 2)
   extern __shared__ __align__(16) double up_smem[];
   UpSmem& sm = *reinterpret_cast<UpSmem*>(up_smem);
   int* ticket = reinterpret_cast<int*>(ws + plan.cnt_off);
-  int* cnt = ticket + 1;
+  int* err = ticket + kErrWord;
+  int* cnt = ticket + kCounters;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   if (tid == 0) {
     sm.node = atomicAdd(ticket, 1);
-    sm.ok = 1;
+    sm.ok = *(volatile int*)err == 0;
   }
   for (int e = tid; e < kNB * kLd; e += kThreads) sm.T[e] = 0.0;
   __syncthreads();
@@ -208,12 +215,12 @@ __global__ void __launch_bounds__(kThreads, 2)
           if ((it & 1023u) != 0) continue;
           asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
           if (t0 == 0) t0 = now;
-          if (now - t0 > 4000000000ull) {
+          if (now - t0 > plan.limit) {
+            atomicCAS(err, 0, kDevTimeoutTree);
             sm.ok = 0;
-            break;
           }
         }
-        *f = 0;  // ready for the next panel
+        if (sm.ok) *f = 0;  // ready for the next panel
       }
       __syncthreads();
       fetch(G);
@@ -736,6 +743,10 @@ int finish_attr() {
 
 long panel_qr_ws_doubles(long m) { return make_plan(m).total; }
 
+const int* panel_error_word(const double* ws) {
+  return reinterpret_cast<const int*>(ws) + kErrWord;  // cnt_off is 0 for every m
+}
+
 int panel_qr_check(long m, long n, long lda) {
   if (n != kNB || m < kNB || (m % kNB) != 0 || lda < m) return EVD_ERR_INVALID_ARG;
   if (m > (1L << 30)) return EVD_ERR_INVALID_ARG;
@@ -795,4 +806,25 @@ extern "C" int evd_panel_qr(long m, long n, double* A, long lda, double* W, long
   if (lwork < evd::panel_qr_ws_doubles(m)) return EVD_ERR_WORKSPACE;
   EVD_TRY(evd::panel_counters_reset(m, work, stream));
   return evd::panel_qr_launch(m, A, lda, work, 1, A, lda, W, ldw, R, ldr, nullptr, 0, stream);
+}
+
+// For the tests: the up-sweep without its first leaf and with waits of `limit`
+// ns (at most 1 s), on a workspace as the last call left it or (fresh) reset;
+// returns the status that a solver would.
+extern "C" int evd_test_tsqr_timeout(long m, double* A, long lda, double* R, double* work,
+                                     int fresh, long limit, cudaStream_t stream) {
+  using namespace evd;
+  EVD_TRY(panel_qr_check(m, kNB, lda));
+  TsqrPlan plan = make_plan(m);
+  if (plan.nlev < 2 || limit > 1000000000) return EVD_ERR_INVALID_ARG;
+  EVD_TRY(finish_attr());
+  if (fresh) EVD_TRY(panel_counters_reset(m, work, stream));
+  const int one = 1;
+  EVD_CUDA_TRY(cudaMemcpyAsync(work, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
+  int nodes = -1;
+  for (int l = 0; l < plan.nlev; ++l) nodes += plan.T[l];
+  plan.limit = (unsigned long long)limit;
+  EVD_TRY(launch_pdl(tsqr_up_kernel, nodes, kThreads, sizeof(UpSmem), stream, plan, A, lda, work,
+                     R, (long)kNB));
+  return read_device_error(panel_error_word(work), stream);
 }

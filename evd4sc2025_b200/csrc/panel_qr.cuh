@@ -11,6 +11,9 @@ int panel_qr_check(long m, long n, long lda);
 // Zero the arrival counters for panels of up to m rows (needed once per
 // workspace; the kernels reset each counter after use).
 int panel_counters_reset(long m, double* ws, cudaStream_t st);
+// The word of the workspace that is not 0 once a wait of a panel has run out
+// (a DeviceError; its R and all that follow from it are NaN).
+const int* panel_error_word(const double* ws);
 // mode 0: A <- explicit thin Q.  mode 1: Yout <- Y, Wout <- W, R <- R and, if
 // Aband != nullptr, the panel of the band matrix (R over zeros) into Aband.
 int panel_qr_launch(long m, double* A, long lda, double* ws, int mode, double* Yout, long ldy,

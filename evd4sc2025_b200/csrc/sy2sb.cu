@@ -85,6 +85,10 @@ static Sy2sbLayout sy2sb_layout(long M, long b, long nb) {
 
 long sy2sb_ws_doubles(long M, long b, long nb) { return sy2sb_layout(M, b, nb).total; }
 
+const int* sy2sb_error_word(const double* work, long M, long b, long nb) {
+  return panel_error_word(work + sy2sb_layout(M, b, nb).panel_off);
+}
+
 // oz != nullptr: the trailing SYR2K is an emulated FP64 product on the
 // integer tensor cores (oz->nmod moduli) instead of the DMMA GEMM.
 int sy2sb(long M, long N, long b, long nb, double* OA, long ldOA, double* dA, long ldA,

@@ -34,7 +34,7 @@ int band_pack(long n, long b, const double* dA, long ldA, double* dSub, long ldS
               cudaStream_t st);
 long chase_iwork_ints(long n);
 int bulge_chase_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, double* d,
-                      double* e, int* iwork, cudaStream_t st);
+                      double* e, int* iwork, const int* before, cudaStream_t st);
 long stedc_ws_doubles(long n);
 int stebz(long n, const double* d, const double* e, double* w, double* work, cudaStream_t st);
 long stedc_ws_ints(long n);
@@ -51,7 +51,9 @@ long q2_flags(long n, long ncols);
 bool chase_pipelined(long n);
 int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, int* iwork,
                      long s0, long s1, int part, cudaStream_t st);
-int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, cudaStream_t st);
+int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, const int* before,
+                  int* iwork, cudaStream_t st);
+const int* sy2sb_error_word(const double* work, long M, long b, long nb);
 int set_identity(long m, long n, double* Q, long ldq, cudaStream_t st);
 long sbr_back_ws_doubles(long n, long b, long nk);
 int wy_merge_slabs(long n, long b, long nk, long ncolsWY, double* dW, long ldW, const double* dY,
@@ -198,6 +200,14 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// The divide and conquer refuses NaN; a wait that ran out before it left that
+// NaN and is the error to report.
+int cause_of(int rc, const int* err_word, cudaStream_t st) {
+  if (rc != EVD_ERR_INVALID_ARG) return rc;
+  EVD_TRY(read_device_error(err_word, st));
+  return rc;
+}
+
 }  // namespace
 
 // err_out != nullptr: the chase's error word is not read here; its address is
@@ -239,14 +249,15 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
     NvtxRange r("evd_b200 bulge chasing");
     EVD_TRY(band_pack(n, b, dA, n, sub, 2 * b, st));
     EVD_CUDA_TRY(cudaMemsetAsync(U, 0, sizeof(double) * n * n, st));
-    EVD_TRY(bulge_chase_async(n, b, sub, 2 * b, U, n, d, e, ich, st));
+    EVD_TRY(bulge_chase_async(n, b, sub, 2 * b, U, n, d, e, ich, sy2sb_error_word(S, n, b, nb),
+                              st));
   }
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[2], st));
   {  // ---- tridiagonal D&C (eigenvectors straight into X) ----
     NvtxRange r("evd_b200 tridiagonal divide and conquer");
-    EVD_TRY(
-        stedc(n, d, e, X, ldX, SW, (long)stedc_ws_doubles(n), ist, (long)stedc_ws_ints(n), st,
-              nullptr));
+    EVD_TRY(cause_of(stedc(n, d, e, X, ldX, SW, (long)stedc_ws_doubles(n), ist,
+                           (long)stedc_ws_ints(n), st, nullptr),
+                     ich + n + 32, st));
   }
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[3], st));
   {  // ---- back transformations ----
@@ -279,7 +290,7 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
     g_timings[5] = ms;
     for (auto& x : ev) cudaEventDestroy(x);
   }
-  // the error word of the bounded waits (chase, stage-2 strips), read once
+  // the error word of the bounded waits (panels, chase, stage-2 strips), read once
   if (err_out) {
     *err_out = ich + n + 32;
     return EVD_SUCCESS;
@@ -427,7 +438,7 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
       EVD_TRY(chase_part_async(n, b, sub, 2 * b, U, n, ich, bounds[i], bounds[i + 1], i, st));
       EVD_CUDA_TRY(cudaEventRecord(evr[i], st));
     }
-    EVD_TRY(chase_tridiag(n, sub, 2 * b, d, e, st));
+    EVD_TRY(chase_tridiag(n, sub, 2 * b, d, e, sy2sb_error_word(S, n, b, nb), ich, st));
   }
   EVD_CUDA_TRY(cudaEventRecord(ev[4], st));
   // ---- the chains (a chase in ranges: range by range behind it) ----
@@ -461,8 +472,10 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
   if (!dc_own) EVD_CUDA_TRY(cudaStreamWaitEvent(st, ev[3], 0));
   {
     NvtxRange r("evd_b200 tridiagonal divide and conquer");
-    EVD_TRY(stedc(n, d, e, W, n, SW, (long)stedc_ws_doubles(n), ist, (long)stedc_ws_ints(n), st,
-                  dc_own ? &ozdc : &oz, dc_own ? ev[3] : nullptr));
+    EVD_TRY(cause_of(stedc(n, d, e, W, n, SW, (long)stedc_ws_doubles(n), ist,
+                           (long)stedc_ws_ints(n), st, dc_own ? &ozdc : &oz,
+                           dc_own ? ev[3] : nullptr),
+                     ich + n + 32, st));
   }
   EVD_CUDA_TRY(cudaEventRecord(ev[6], st));
   // ---- side A: the products (emulated, the main integer workspace; the Q1
@@ -571,7 +584,8 @@ static int values_core(long n, long b, long nb, const double* A, long lda, doubl
                 (long)sy2sb_ws_doubles(n, b, nb), st, nullptr));
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[1], st));
   EVD_TRY(band_pack(n, b, dA, n, sub, 2 * b, st));
-  EVD_TRY(bulge_chase_async(n, b, sub, 2 * b, nullptr, n, d, e, ich, st));
+  EVD_TRY(bulge_chase_async(n, b, sub, 2 * b, nullptr, n, d, e, ich,
+                            sy2sb_error_word(S, n, b, nb), st));
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[2], st));
   EVD_TRY(stebz(n, d, e, w, SW, st));
   if (timed) {

@@ -84,6 +84,10 @@ int evd_syr2k_lower_mirror(long n, long k, double alpha, const double* A, long l
 
 /* ---- Stage 1: full -> band (ZY) ---------------------------------------- */
 
+/* The three calls of this stage do not synchronise.  The panel's tree waits
+ * between blocks, 4 s at most; a wait that runs out leaves NaN in R (and in the
+ * band).  The solvers below report it as EVD_ERR_TIMEOUT. */
+
 /* Workspace (in doubles) needed by evd_tsqr / evd_panel_qr for an m x n panel. */
 long evd_panel_qr_work_size(long m, long n);
 

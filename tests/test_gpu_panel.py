@@ -48,3 +48,30 @@ def test_panel_rejects_bad_shapes(cuda, evdlib):
     A = evdlib.to_cm(torch.randn(100, 32, dtype=torch.float64), device=cuda)  # m % 32 != 0
     with pytest.raises(evdlib.EvdError):
         evdlib.panel_qr(A)
+
+
+@pytest.mark.parametrize("m", [256, 544, 4128])
+def test_a_tree_wait_that_runs_out_is_reported_and_stays_visible(cuda, evdlib, m):
+    """The first leaf never runs: its parent's wait ends with a status and NaN,
+    and so does a panel on the counters that this leaves behind; a call that
+    resets them is right again."""
+    import ctypes as C
+    A = torch.from_numpy(np.random.default_rng(m).standard_normal((m, 32)))
+    work = torch.zeros(evdlib.lib().evd_panel_qr_work_size(m, 32), dtype=torch.float64,
+                       device=cuda)
+    for fresh in (1, 0):
+        Ad = evdlib.to_cm(A, device=cuda)
+        R = torch.zeros(32, 32, dtype=torch.float64, device=cuda)
+        torch.cuda.synchronize()
+        rc = evdlib.lib().evd_test_tsqr_timeout(
+            C.c_long(m), C.c_void_p(Ad.data_ptr()), C.c_long(m), C.c_void_p(R.data_ptr()),
+            C.c_void_p(work.data_ptr()), C.c_int(fresh), C.c_long(2000000), None)
+        assert rc == -3  # EVD_ERR_TIMEOUT
+        assert torch.isnan(torch.triu(R.t())).sum() == 32 * 33 // 2
+    Ad, R = evdlib.to_cm(A, device=cuda), evdlib.empty_cm(32, 32, device=cuda)
+    rc = evdlib.lib().evd_tsqr(m, 32, C.c_void_p(Ad.data_ptr()), m, C.c_void_p(R.data_ptr()), 32,
+                               C.c_void_p(work.data_ptr()), work.numel(), None)
+    torch.cuda.synchronize()
+    assert rc == 0
+    Rr = O.tsqr(A.numpy())[1]
+    assert np.abs(R.cpu().numpy() - Rr).max() <= 1e-12 * np.abs(Rr).max()
