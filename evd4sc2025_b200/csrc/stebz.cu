@@ -40,13 +40,18 @@ __host__ __device__ __forceinline__ auto* rows_of(T* ws) {
 __global__ void stebz_prep_kernel(long n, const double* __restrict__ d,
                                   const double* __restrict__ e, double* __restrict__ ws) {
   // ws[0] = scale = max |d|, |e|; ws[1] = gl, ws[2] = gu (Gershgorin, scaled);
-  // ws[3] = pivmin; then rows(ws)[i] = (d_i/scale, e_{i-1}^2/scale^2)
+  // ws[3] = pivmin; then rows(ws)[i] = (d_i/scale, e_{i-1}^2/scale^2).
+  // fmax drops NaN: an entry that is not finite makes gl and gu NaN, and with
+  // them every eigenvalue
   __shared__ double red[3][32];
   double m = 0.0;
+  bool bad = false;
   for (long i = threadIdx.x; i < n; i += blockDim.x) {
-    m = fmax(m, fabs(d[i]));
-    if (i < n - 1) m = fmax(m, fabs(e[i]));
+    const double a = fabs(d[i]), b = (i < n - 1) ? fabs(e[i]) : 0.0;
+    m = fmax(m, fmax(a, b));
+    bad |= !isfinite(a) || !isfinite(b);
   }
+  bad = __syncthreads_or(bad) != 0;
   m = warp_max(m);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) red[0][w] = m;
@@ -86,8 +91,8 @@ __global__ void stebz_prep_kernel(long n, const double* __restrict__ d,
       c = fmax(c, red[2][k]);
     }
     const double pad = 2.0 * 2.220446049250313e-16 * fmax(fabs(a), fabs(b)) * (double)n + 1e-300;
-    ws[1] = a - pad;
-    ws[2] = b + pad;
+    ws[1] = bad ? __longlong_as_double(0x7ff8000000000000ll) : a - pad;
+    ws[2] = bad ? __longlong_as_double(0x7ff8000000000000ll) : b + pad;
     ws[3] = 2.2250738585072014e-308 * fmax(1.0, c);  // LAPACK pivmin = safmin * max(1, e^2)
   }
 }

@@ -176,7 +176,8 @@ int evd_stedc(long n, double* d, double* e, double* Z, long ldz, double* work, l
  * vectors: Sturm-count multisection with the pivot rule of LAPACK dstebz.  The
  * eigenvalues-only counterpart of the reference's LAPACKE_dstedc('I') call
  * (src/EVD/myEVD.cu:529), which always forms vectors.  work: evd_stebz_work_size
- * doubles.  d and e are not modified. */
+ * doubles.  d and e are not modified.  Entries that are not finite give NaN in
+ * every w. */
 long evd_stebz_work_size(long n);
 int evd_stebz(long n, const double* d, const double* e, double* w, double* work, long lwork,
               cudaStream_t stream);

@@ -107,3 +107,27 @@ def test_stebz_vanishing_terms(cuda, evdlib, kind, n):
     w = evdlib.stebz(torch.from_numpy(d).to(cuda), torch.from_numpy(e).to(cuda)).cpu().numpy()
     w_ref = O.tridiag_eig(d, e)[0]
     assert np.abs(w - w_ref).max() <= 1e-13 * max(np.abs(w_ref).max(), 1e-300) * np.sqrt(n)
+
+
+@pytest.mark.parametrize("n", [2, 9, 100, 1500])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["d", "e", "all"])
+def test_stebz_passes_non_finite_entries_on(cuda, evdlib, n, bad, where):
+    rng = np.random.default_rng(n)
+    d, e = rng.standard_normal(n), rng.standard_normal(n - 1)
+    if where == "all":
+        d[:], e[:] = bad, bad
+    else:
+        (d if where == "d" else e)[(n - 1) // 2 if where == "d" else (n - 2) // 2] = bad
+    w = evdlib.stebz(torch.from_numpy(d).to(cuda), torch.from_numpy(e).to(cuda))
+    assert torch.isnan(w).all()
+
+
+@pytest.mark.parametrize("n,nb", [(100, 64), (64, 32), (1000, 256)])
+@pytest.mark.parametrize("at", [(0, 0), (5, 3), (-1, 0), (-1, -1)])
+def test_values_of_a_matrix_with_nan(cuda, evdlib, n, nb, at):
+    """A NaN in A reaches the eigenvalues; it does not end as zeros."""
+    A = O.sym_gaussian(n, n)
+    A[at] = A[at[::-1]] = np.nan
+    w = evdlib.syevd_values(evdlib.to_cm(torch.from_numpy(A), device=cuda), 32, nb)
+    assert torch.isnan(w).all()
