@@ -341,7 +341,7 @@ long chase_iwork_ints(long n) { return n + 64 + chase_pipe_ints(n); }
 // first sweep starts when the previous sweep has reached the end of the band,
 // not 2b rows after its start.
 int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, int* iwork,
-                     long s0, long s1, int part, cudaStream_t st) {
+                     long s0, long s1, int part, int form, cudaStream_t st) {
   if (n < 0 || b != kBW || ldSub != 2 * b || (dU && n > 0 && ldU < n)) return EVD_ERR_INVALID_ARG;
   if (((uintptr_t)dSub & 15u) != 0) return EVD_ERR_INVALID_ARG;
   if (n > (1L << 30)) return EVD_ERR_INVALID_ARG;
@@ -355,7 +355,8 @@ int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long 
   s1 = std::min(s1, n - 2);
   if (s1 > s0) {
     bool used = false;
-    EVD_TRY(launch_chase_pipe(n, dSub, dU, ldU, err, iwork + n + 64, s0, s1, st, &used));
+    if (form == kChaseAuto)
+      EVD_TRY(launch_chase_pipe(n, dSub, dU, ldU, err, iwork + n + 64, s0, s1, st, &used));
     if (used) return EVD_SUCCESS;
     // enough CTAs for the pipeline's concurrency (a sweep starts every 3 steps
     // and lasts about n/b steps), bounded by the GPU's resident capacity
@@ -387,13 +388,14 @@ int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, 
 // The tile copies need ldSub == 2b exactly (contiguous band columns) and a
 // 16-byte aligned dSub.
 int bulge_chase_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU,
-                      double* d, double* e, int* iwork, const int* before, cudaStream_t st) {
+                      double* d, double* e, int* iwork, const int* before, int form,
+                      cudaStream_t st) {
   if (n < 0 || b != kBW || ldSub != 2 * b || (dU && n > 0 && ldU < n)) return EVD_ERR_INVALID_ARG;
   if (((uintptr_t)dSub & 15u) != 0) return EVD_ERR_INVALID_ARG;
   if (n > (1L << 30)) return EVD_ERR_INVALID_ARG;
   if (n == 0) return EVD_SUCCESS;
   if (!dSub || !d || !iwork || (n > 1 && !e)) return EVD_ERR_INVALID_ARG;  // dU may be NULL
-  EVD_TRY(chase_part_async(n, b, dSub, ldSub, dU, ldU, iwork, 0, n - 2, 0, st));
+  EVD_TRY(chase_part_async(n, b, dSub, ldSub, dU, ldU, iwork, 0, n - 2, 0, form, st));
   return chase_tridiag(n, dSub, ldSub, d, e, before, iwork, st);
 }
 
@@ -421,7 +423,8 @@ extern "C" long evd_bulge_chase_iwork_size(long n) {
 
 extern "C" int evd_bulge_chase(long n, long b, double* dSub, long ldSub, double* dU, long ldU,
                                double* d, double* e, int* iwork, cudaStream_t stream) {
-  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iwork, nullptr, stream);
+  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iwork, nullptr, evd::kChaseAuto,
+                                  stream);
   if (rc != EVD_SUCCESS || n <= 2) return rc;
   return evd::read_device_error(iwork + n + 32, stream);
 }
@@ -487,7 +490,16 @@ extern "C" int evd_bulge_chase_noalloc(long n, long b, double* dSub, long ldSub,
   EVD_TRY(evd::chase_noalloc_scratch(&iw));
   // bulge_chase_async clears the flags, ticket and error word of the scratch
   // (cudaMemsetAsync) before every launch, so a call never sees stale state.
-  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iw, nullptr, stream);
+  int rc = evd::bulge_chase_async(n, b, dSub, ldSub, dU, ldU, d, e, iw, nullptr, evd::kChaseAuto, stream);
   if (rc != EVD_SUCCESS || n <= 2) return rc;
   return evd::read_device_error(iw + n + 32, stream);
+}
+
+// For the tests: evd_bulge_chase by the given form (a ChaseForm), with the error
+// word of the stages before it.
+extern "C" int evd_test_bulge_chase(long n, double* dSub, double* dU, long ldU, double* d,
+                                    double* e, int* iwork, const int* before, int form,
+                                    cudaStream_t stream) {
+  EVD_TRY(evd::bulge_chase_async(n, 32, dSub, 64, dU, ldU, d, e, iwork, before, form, stream));
+  return evd::read_device_error(iwork + n + 32, stream);
 }

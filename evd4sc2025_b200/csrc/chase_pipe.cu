@@ -612,9 +612,10 @@ long chase_pipe_ints(long n) {
   return ctas * (long)(sizeof(Boundary) / sizeof(int)) + 4;
 }
 
-// Whether the whole chase of order n runs as one pipeline launch.
-bool chase_pipelined(long n) {
-  const long most = std::min(device_sm_count(), kMaxPipeCtas);
+// Whether the whole chase of order n runs as one pipeline launch on a device
+// with `sms` SMs.
+bool chase_pipelined(long n, int sms) {
+  const long most = std::min(sms, kMaxPipeCtas);
   return n < 3 || (n - 2) / kPB + 1 <= most * kSlB;
 }
 

@@ -55,6 +55,10 @@ enum DeviceError : int {
   kDevTimeoutStrips = 5,
 };
 
+// Which kernel runs a chase: the pipeline where it fits, or (the tests, at orders
+// where the pipeline would run) always the kernel with ticketed sweeps.
+enum ChaseForm : int { kChaseAuto = 0, kChaseTicketed = 1 };
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);

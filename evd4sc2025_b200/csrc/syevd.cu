@@ -34,7 +34,7 @@ int band_pack(long n, long b, const double* dA, long ldA, double* dSub, long ldS
               cudaStream_t st);
 long chase_iwork_ints(long n);
 int bulge_chase_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, double* d,
-                      double* e, int* iwork, const int* before, cudaStream_t st);
+                      double* e, int* iwork, const int* before, int form, cudaStream_t st);
 long stedc_ws_doubles(long n);
 int stebz(long n, const double* d, const double* e, double* w, double* work, cudaStream_t st);
 long stedc_ws_ints(long n);
@@ -48,9 +48,9 @@ int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, 
                    long ldX, double* tbuf, int* flags, int* err, long h0, long h1,
                    long ident_k, cudaStream_t st);
 long q2_flags(long n, long ncols);
-bool chase_pipelined(long n);
+bool chase_pipelined(long n, int sms);
 int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long ldU, int* iwork,
-                     long s0, long s1, int part, cudaStream_t st);
+                     long s0, long s1, int part, int form, cudaStream_t st);
 int chase_tridiag(long n, const double* dSub, long ldSub, double* d, double* e, const int* before,
                   int* iwork, cudaStream_t st);
 const int* sy2sb_error_word(const double* work, long M, long b, long nb);
@@ -88,6 +88,7 @@ struct MixedOpts {
   uint8_t* oz_q1;  // the Q1 formation's own integer workspace, or nullptr
   long oz_q1_bytes;
   double* split_buf;  // an n x n buffer for the second stage-2 chain, or nullptr
+  int chase_form;     // a ChaseForm
 };
 
 // Orders up to this one get a separate integer workspace for the divide and
@@ -250,7 +251,7 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
     EVD_TRY(band_pack(n, b, dA, n, sub, 2 * b, st));
     EVD_CUDA_TRY(cudaMemsetAsync(U, 0, sizeof(double) * n * n, st));
     EVD_TRY(bulge_chase_async(n, b, sub, 2 * b, U, n, d, e, ich, sy2sb_error_word(S, n, b, nb),
-                              st));
+                              kChaseAuto, st));
   }
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[2], st));
   {  // ---- tridiagonal D&C (eigenvectors straight into X) ----
@@ -300,37 +301,29 @@ static int syevd_core(long n, long b, long nb, const double* A, long lda, double
 
 size_t syevd_ws_bytes(long n, long b, long nb) { return layout(n, b, nb).bytes; }
 
-// Sweep ranges of a chase too long for the pipeline kernel (n > 33000 or so):
-// [0, 512), [512, 1536), ... doubling up to k, then max(2048, (n - 2 - k) / 16)
-// sweeps each, the last one ending at sweep n - 2, so that stage 2 can follow
-// one range behind.  k = 0: no lower part.  Returns the number of ranges r (at
-// most 32); range i is [bounds[i], bounds[i+1]).
-static int chase_ranges(long n, long k, long bounds[34]) {
-  const long S = std::max(n - 2, 0L);
-  int c = 0;
-  bounds[c++] = 0;
-  long s = 0, len = 512;
-  while (s + len < k) {
-    s += len;
-    bounds[c++] = s;
-    len *= 2;
-  }
-  if (k > 0 && k < S) bounds[c++] = k;
-  s = std::max(k, 0L);
-  const long step = std::max(2048L, ((S - s) / 16 + 7) / 8 * 8);
-  while (s + step < S) {
-    s += step;
-    bounds[c++] = s;
-  }
-  bounds[c] = S;
-  return c;
-}
+// How the mixed form runs its chase and its stage-2 chains (see below).
+struct ChainPlan {
+  bool split;       // two chains from the identity, below and from sweep k
+  long k;
+  int nr;           // sweep ranges of the chase: [bounds[i], bounds[i + 1])
+  long bounds[34];
+};
 
-// The whole chase as one range.
-static int one_range(long n, long bounds[34]) {
-  bounds[0] = 0;
-  bounds[1] = std::max(n - 2, 0L);
-  return 1;
+// A chase that is one launch (chase_pipelined) is one range, and with a buffer
+// for it the reflectors are accumulated in two chains.  A longer chase (n above
+// 224 per SM, 33152 on B200) runs in ranges of max(2048, (n - 2) / 16) sweeps, a
+// multiple of 8, and one chain follows it a range behind: beside the slower
+// chase a second chain has nothing to gain.
+ChainPlan chain_plan(long n, bool buffer, bool pipelined) {
+  ChainPlan p{};
+  const long S = std::max(n - 2, 0L);
+  p.split = buffer && pipelined && n > 64;
+  p.k = p.split ? std::max(8L, (long)(0.293 * (double)n) / 8 * 8) : 0;
+  const long step = pipelined ? std::max(S, 1L) : std::max(2048L, (S / 16 + 7) / 8 * 8);
+  p.bounds[p.nr++] = 0;
+  for (long s = step; s < S; s += step) p.bounds[p.nr++] = s;
+  p.bounds[p.nr] = S;
+  return p;
 }
 
 // The mixed form.  Q2^T = B A with A = the reflectors of the sweeps [0, k) and
@@ -379,8 +372,12 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
   // they do not fit and the stage-2 kernel rebuilds them itself
   double* tbuf = ((size_t)q2_tbuf_doubles(n) <= (size_t)n * n) ? OA : nullptr;
   double* XA = mx->split_buf;  // chain A, then Q^T
-  const bool split = XA != nullptr && n > 64;
-  const long k = split ? std::max(8L, (long)(0.293 * (double)n) / 8 * 8) : 0;
+  const ChainPlan plan = chain_plan(
+      n, XA != nullptr, mx->chase_form == kChaseAuto && chase_pipelined(n, device_sm_count()));
+  const bool split = plan.split;
+  const long k = plan.k;
+  const int nr = plan.nr;
+  const long* bounds = plan.bounds;
   SideStream sideA, sideB, sideC;
   EVD_TRY(sideA.init(timed != 0));
   EVD_TRY(sideB.init(timed != 0));
@@ -392,8 +389,6 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
   // sideB.ev[i]: chase range i done
   cudaEvent_t* ev = sideA.ev;
   cudaEvent_t* evr = sideB.ev;
-  long bounds[34];
-  const int nr = chase_pipelined(n) ? one_range(n, bounds) : chase_ranges(n, k, bounds);
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[0], st));
   {
     NvtxRange r("evd_b200 sy2sb (emulated trailing update)");
@@ -435,7 +430,8 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
     NvtxRange r("evd_b200 bulge chasing");
     EVD_CUDA_TRY(cudaMemsetAsync(U, 0, sizeof(double) * n * n, st));
     for (int i = 0; i < nr; ++i) {
-      EVD_TRY(chase_part_async(n, b, sub, 2 * b, U, n, ich, bounds[i], bounds[i + 1], i, st));
+      EVD_TRY(chase_part_async(n, b, sub, 2 * b, U, n, ich, bounds[i], bounds[i + 1], i,
+                               mx->chase_form, st));
       EVD_CUDA_TRY(cudaEventRecord(evr[i], st));
     }
     EVD_TRY(chase_tridiag(n, sub, 2 * b, d, e, sy2sb_error_word(S, n, b, nb), ich, st));
@@ -452,14 +448,17 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
     const bool fits = n < 64L * device_sm_count() && q2_flags(n, n) > 0 &&
                       q2_flags(n, n) <= 2 * n * nb;
     int* fl[2] = {fits ? (int*)Z : nullptr, fits ? (int*)R : nullptr};
-    for (int i = 0; i < nr; ++i) {
-      EVD_CUDA_TRY(cudaStreamWaitEvent(sa, evr[i], 0));
-      EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, fl[0], ich + n + 32,
-                             bounds[i], split ? k : bounds[i + 1], 0, sa));
-      if (split) {
-        EVD_CUDA_TRY(cudaStreamWaitEvent(sc, evr[i], 0));
-        EVD_TRY(q2_apply_range(true, n, n, U, n, X, ldX, tbuf, fl[1], ich + n + 32, k,
-                               bounds[i + 1], k, sc));
+    if (split) {  // the chase is one range
+      EVD_CUDA_TRY(cudaStreamWaitEvent(sa, evr[0], 0));
+      EVD_CUDA_TRY(cudaStreamWaitEvent(sc, evr[0], 0));
+      EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, fl[0], ich + n + 32, 0, k, 0, sa));
+      EVD_TRY(q2_apply_range(true, n, n, U, n, X, ldX, tbuf, fl[1], ich + n + 32, k, bounds[1],
+                             k, sc));
+    } else {
+      for (int i = 0; i < nr; ++i) {
+        EVD_CUDA_TRY(cudaStreamWaitEvent(sa, evr[i], 0));
+        EVD_TRY(q2_apply_range(true, n, n, U, n, PA, ldPA, tbuf, fl[0], ich + n + 32, bounds[i],
+                               bounds[i + 1], 0, sa));
       }
     }
   }
@@ -585,7 +584,7 @@ static int values_core(long n, long b, long nb, const double* A, long lda, doubl
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[1], st));
   EVD_TRY(band_pack(n, b, dA, n, sub, 2 * b, st));
   EVD_TRY(bulge_chase_async(n, b, sub, 2 * b, nullptr, n, d, e, ich,
-                            sy2sb_error_word(S, n, b, nb), st));
+                            sy2sb_error_word(S, n, b, nb), kChaseAuto, st));
   if (timed) EVD_CUDA_TRY(cudaEventRecord(ev[2], st));
   EVD_TRY(stebz(n, d, e, w, SW, st));
   if (timed) {
@@ -740,7 +739,7 @@ size_t syevd_mixed_ws_bytes(long n, long b, long nb, int nmod, int refine_iters)
 
 int syevd_mixed(long n, long b, long nb, const double* A, long lda, double* w, double* X,
                 long ldX, int nmod, int refine_iters, int moduli_update, void* work,
-                long lwork_bytes, int timed, cudaStream_t st) {
+                long lwork_bytes, int timed, cudaStream_t st, int chase_form = kChaseAuto) {
   if (!shape_ok(n, b, nb)) return EVD_ERR_INVALID_ARG;
   if (nmod < kOzMinMod || nmod > kOzMaxMod || refine_iters < 0 || refine_iters > 16 ||
       moduli_update < kOzMinMod || moduli_update > kOzFp64Mod)
@@ -757,7 +756,8 @@ int syevd_mixed(long n, long b, long nb, const double* A, long lda, double* w, d
   const long ozn = mixed_oz_bytes(np, nb, nmod, refine_iters);
   const MixedExtra xt = mixed_extra(np, nb, nmod);
   uint8_t* xb = reinterpret_cast<uint8_t*>(((uintptr_t)(ozb + ozn) + 255) & ~(uintptr_t)255);
-  MixedOpts mx{nmod, refine_iters, moduli_update, ozb, ozn, nullptr, 0, nullptr, 0, nullptr};
+  MixedOpts mx{nmod, refine_iters, moduli_update, ozb, ozn, nullptr, 0, nullptr, 0, nullptr,
+               chase_form};
   if (full && xt.total > 0) {
     mx.oz_dc = xb;
     mx.oz_dc_bytes = xt.dc;
@@ -929,4 +929,27 @@ extern "C" double evd_syevd_last_refine_ms(void) { return evd::g_refine_ms; }
 
 extern "C" void evd_syevd_mixed_last_timings(double out_ms[8]) {
   for (int i = 0; i < 8; ++i) out_ms[i] = evd::g_mixed[i];
+}
+
+// For the tests: the mixed solve as on a device whose SMs cannot hold the chase
+// pipeline (the chase in ranges by the ticketed kernel).
+extern "C" int evd_test_syevd_mixed_ranges(long n, long nb, const double* A, long lda, double* w,
+                                           double* X, long ldX, int moduli, void* work,
+                                           long lwork_bytes, cudaStream_t stream) {
+  try {
+    return evd::syevd_mixed(n, 32, nb, A, lda, w, X, ldX, moduli, 0, moduli, work, lwork_bytes, 0,
+                            stream, evd::kChaseTicketed);
+  } catch (...) {
+    return EVD_ERR_HOST;
+  }
+}
+
+// For the tests: out = {split, k, ranges, their bounds} of an order on a device
+// with `sms` SMs; `buffer`: there is one for the second chain.
+extern "C" void evd_test_chain_plan(long n, int buffer, int sms, long out[37]) {
+  const evd::ChainPlan p = evd::chain_plan(n, buffer != 0, evd::chase_pipelined(n, sms));
+  out[0] = p.split;
+  out[1] = p.k;
+  out[2] = p.nr;
+  for (int i = 0; i <= p.nr; ++i) out[3 + i] = p.bounds[i];
 }

@@ -99,3 +99,51 @@ def test_chase_is_an_orthogonal_similarity(cuda, evdlib, n):
     # backward stable: a few units of rounding per reflector that a row meets
     norm2 = 2.0 * 65 ** 0.5  # of a random band matrix, from above to within a factor of 2
     assert (BQZ - QTZ).norm() <= 8e-13 * norm2 * Z.norm()
+
+
+def _chase(evdlib, cuda, band, form, before=None):
+    import ctypes as C
+    n = band.shape[0]
+    sub, U = band.clone(), torch.zeros(n, n, dtype=torch.float64, device=cuda)
+    d = torch.empty(n, dtype=torch.float64, device=cuda)
+    e = torch.empty(n, dtype=torch.float64, device=cuda)
+    iw = torch.empty(evdlib.lib().evd_bulge_chase_iwork_size(n) // 4, dtype=torch.int32,
+                     device=cuda)
+    torch.cuda.synchronize()
+    rc = evdlib.lib().evd_test_bulge_chase(
+        C.c_long(n), C.c_void_p(sub.data_ptr()), C.c_void_p(U.data_ptr()), C.c_long(n),
+        C.c_void_p(d.data_ptr()), C.c_void_p(e.data_ptr()), C.c_void_p(iw.data_ptr()),
+        C.c_void_p(before.data_ptr() if before is not None else None), form, None)
+    torch.cuda.synchronize()
+    return rc, d, e[: n - 1], U
+
+
+@pytest.mark.parametrize("n", [3, 34, 65, 100, 257, 512, 1100, 2200, 4200])
+def test_ticketed_chase_agrees_with_the_pipeline(cuda, evdlib, n):
+    """The kernel of orders beyond the pipeline, at orders that reach both."""
+    g = torch.Generator(device=cuda).manual_seed(n)
+    band = torch.zeros(n, 64, dtype=torch.float64, device=cuda)
+    for o in range(min(33, n)):
+        band[: n - o, o] = torch.randn(n - o, generator=g, dtype=torch.float64, device=cuda)
+    rc, d, e, U = _chase(evdlib, cuda, band, 0)
+    rt, dt, et, Ut = _chase(evdlib, cuda, band, 1)
+    assert rc == 0 and rt == 0
+    B = np.zeros((n, n))
+    for o in range(min(33, n)):
+        v = band[: n - o, o].cpu().numpy()
+        B += np.diag(v, -o) + (np.diag(v, o) if o else 0)
+    w = np.linalg.eigvalsh(B)
+    for a, b in ((d, e), (dt, et)):
+        wt = eigvalsh_tridiagonal(a.cpu().numpy(), b.cpu().numpy())
+        assert np.abs(wt - w).max() <= 8e-12 * np.abs(w).max()
+    # the first sweeps, where rounding has not grown yet, reflector by reflector
+    assert (U[: min(n, 64), :8] - Ut[: min(n, 64), :8]).abs().max() <= 1e-10
+
+
+def test_chase_reports_an_error_of_the_stages_before_it(cuda, evdlib):
+    band = torch.zeros(100, 64, dtype=torch.float64, device=cuda)
+    band[:, 0] = 1.0
+    word = torch.tensor([2], dtype=torch.int32, device=cuda)
+    assert _chase(evdlib, cuda, band, 0, word)[0] == -3  # EVD_ERR_TIMEOUT
+    word.zero_()
+    assert _chase(evdlib, cuda, band, 0, word)[0] == 0

@@ -132,3 +132,27 @@ def test_mixed_minimal_workspace_one_chain(cuda, evdlib, n, nb, moduli, iters):
                                       Xd.data_ptr(), n, moduli, iters, 14, short.data_ptr(),
                                       lmin - 1, 0, None)
     assert rc == -5  # EVD_ERR_WORKSPACE
+
+
+@pytest.mark.parametrize("n,nb", [(1000, 256), (4500, 512)])
+def test_mixed_with_the_chase_in_ranges(cuda, evdlib, n, nb):
+    """The schedule of a device whose SMs cannot hold the chase pipeline: one
+    chain behind a chase in ranges, although the buffer for two is there."""
+    import ctypes as C
+    A = O.sym_gaussian(n, seed=n)
+    Ad = evdlib.to_cm(torch.from_numpy(A), device=cuda)
+    w = torch.empty(n, dtype=torch.float64, device=cuda)
+    X = evdlib.empty_cm(n, n, device=cuda)
+    nbytes = evdlib.lib().evd_syevd_mixed_work_size(n, 32, nb, 14, 0)
+    work = torch.empty(nbytes, dtype=torch.uint8, device=cuda)
+    torch.cuda.synchronize()
+    rc = evdlib.lib().evd_test_syevd_mixed_ranges(
+        C.c_long(n), C.c_long(nb), C.c_void_p(Ad.data_ptr()), C.c_long(n),
+        C.c_void_p(w.data_ptr()), C.c_void_p(X.data_ptr()), C.c_long(n), 14,
+        C.c_void_p(work.data_ptr()), C.c_long(nbytes), None)
+    torch.cuda.synchronize()
+    assert rc == 0
+    res, orth = evdlib.check_eig(Ad, w, X)
+    assert res <= 1e-13 and orth <= 1e-13, (res, orth)
+    wp, _ = evdlib.syevd(Ad, 32, nb)
+    assert (w - wp).abs().max() <= 1e-13 * np.linalg.norm(A, 2)

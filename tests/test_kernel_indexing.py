@@ -152,6 +152,26 @@ def test_stage2_two_chains_from_the_identity():
         assert not B[:k + 1, k + 1:].any() and not B[k + 1:, :k + 1].any()
 
 
+def test_mixed_chain_plan_applies_every_sweep_once(evdlib):
+    """The schedule of the mixed solve on devices with few SMs (a partition of
+    a GPU), where an order may have the buffer for two chains and a chase too
+    long for the pipeline."""
+    import ctypes as C
+    out = (C.c_long * 37)()
+    for sms in (8, 28, 60, 109, 148):
+        for n in (64, 96, 1024, 1792, 6272, 6304, 13440, 24416, 24576, 32768, 34816, 65536):
+            for buffer in (0, 1):
+                evdlib.lib().evd_test_chain_plan(C.c_long(n), buffer, sms, out)
+                split, k, nr, bounds = out[0], out[1], out[2], list(out[3:4 + out[2]])
+                assert 1 <= nr <= 32 and bounds[0] == 0 and bounds[-1] == n - 2
+                assert all(a < b for a, b in zip(bounds, bounds[1:]))
+                assert all(b % 8 == 0 for b in bounds[:-1]) and k % 8 == 0
+                pipelined = (n - 2) // 32 + 1 <= 7 * min(sms, 160)
+                assert (nr == 1) if pipelined else not split
+                assert split == (buffer and pipelined and n > 64)
+                assert nr == 1 and 0 < k < n - 2 if split else k == 0
+
+
 # ---------------------------------------------------------------------------
 # Panel QR tile factorisation (evd4sc2025_b200/csrc/panel_qr.cu, tile_factor):
 # warp w owns columns w, w + 8, ...; the owner of column j + 1 publishes
