@@ -449,7 +449,10 @@ __global__ void __launch_bounds__(kDefMax) merge_deflate_kernel(LevelArgs a) {
     const unsigned lb = __ballot_sync(0xffffffffu, live);
     if (lane == 0) s_live[wid] = lb;
     __syncthreads();
-    if (s_bad) return;
+    if (s_bad) {  // the host sizes the level by the descriptor: leave an empty one
+      if (tid < D_PAD) d_[tid] = 0;
+      return;
+    }
     // the neighbouring live entries of the chunk (0: the pending one; -1: none)
     int prev = have ? 0 : -1, next = -1;
     {
@@ -1158,4 +1161,29 @@ extern "C" long evd_stedc_iwork_size(long n) { return evd::stedc_ws_ints(n < 0 ?
 extern "C" int evd_stedc(long n, double* d, double* e, double* Z, long ldz, double* work,
                          long lwork, int* iwork, long liwork, cudaStream_t stream) {
   return evd::stedc(n, d, e, Z, ldz, work, lwork, iwork, liwork, stream, nullptr, nullptr);
+}
+
+// For the tests: the deflation of one merge of N entries, ds and zs in the order
+// `perm`.  dwork: 7 N + 1 doubles, iwork: 8 N + 9 ints; desc gets its descriptor.
+extern "C" int evd_test_merge_deflate(int N, double* ds, double* zs, int* perm, double rho,
+                                      double* dwork, int* iwork, int* desc,
+                                      cudaStream_t stream) {
+  using namespace evd;
+  LevelArgs a{};
+  a.N = N;
+  a.n1 = N / 2;
+  a.n2 = N - a.n1;
+  a.nm = 1;
+  a.ds = ds;
+  a.zs = zs;
+  a.perm = perm;
+  double** dp[] = {&a.dK, &a.zK, &a.dD, &a.rc, &a.rs, &a.zv, &a.dw, &a.rho};
+  for (double** p : dp) *p = dwork, dwork += N;
+  int** ip[] = {&a.colK, &a.typK, &a.pT, &a.pB, &a.colD, &a.rA, &a.rB, &a.org, &a.err};
+  for (int** p : ip) *p = iwork, iwork += N;
+  a.desc = desc;
+  EVD_CUDA_TRY(cudaMemsetAsync(a.err, 0, sizeof(int), stream));
+  EVD_CUDA_TRY(cudaMemcpyAsync(a.rho, &rho, sizeof(double), cudaMemcpyHostToDevice, stream));
+  EVD_TRY(launch_pdl(merge_deflate_kernel, 1, std::min(kDefMax, (N + 31) / 32 * 32), 0, stream, a));
+  return read_device_error(a.err, stream);
 }

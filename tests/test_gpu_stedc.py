@@ -102,3 +102,26 @@ def test_stedc_rotation_runs(cuda, evdlib, n, kind):
         d, e = rng.standard_normal(n), rng.standard_normal(n - 1)
         d[n // 3: 2 * n // 3], e[n // 3: 2 * n // 3] = 0.25, 1e-17
     _check(cuda, evdlib, d, e)
+
+
+@pytest.mark.parametrize("N", [40, 1500])
+def test_deflation_of_a_broken_order_leaves_an_empty_descriptor(cuda, evdlib, N):
+    """The host sizes a level's work by the descriptors, so one that a broken
+    merge order stops must not keep what was in memory."""
+    import ctypes as C
+    rng = np.random.default_rng(N)
+    ds = torch.from_numpy(np.sort(rng.standard_normal(N))).to(cuda)
+    zs = torch.from_numpy(rng.standard_normal(N) / np.sqrt(N)).to(cuda)
+    dwork = torch.zeros(7 * N + 1, dtype=torch.float64, device=cuda)
+    iwork = torch.zeros(8 * N + 9, dtype=torch.int32, device=cuda)
+    for broken in (False, True):
+        perm = torch.arange(N, dtype=torch.int32, device=cuda)
+        if broken:
+            perm[N - 3] = N
+        desc = torch.full((8,), 1 << 28, dtype=torch.int32, device=cuda)
+        torch.cuda.synchronize()
+        rc = evdlib.lib().evd_test_merge_deflate(
+            N, *(C.c_void_p(t.data_ptr()) for t in (ds, zs, perm)), C.c_double(1.0),
+            *(C.c_void_p(t.data_ptr()) for t in (dwork, iwork, desc)), None)
+        got = desc.tolist()[:6]
+        assert (rc == -1 and got == [0] * 6) if broken else (rc == 0 and got[0] + got[4] == N)
