@@ -1,5 +1,6 @@
 // Stage 2: band -> tridiagonal bulge chasing: the entry points, and the
-// kernel for orders beyond the reach of the pipeline kernel (chase_pipe.cu).
+// kernel for orders beyond the reach of the pipeline kernel (chase_pipe.cu), and
+// for its launches whose CTAs did not get their SMs in time.
 //
 // Algorithm (same reflectors, same storage as chasing_kernel_one_timeV10,
 // util/inc/bugle_chasingV10.h:21-392): sweep s (s = 0..n-3) annihilates column
@@ -36,8 +37,8 @@
 namespace evd {
 
 long chase_pipe_ints(long n);
-int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* msg, long s0,
-                      long s1, cudaStream_t st, bool* used);
+int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* msg, int* gate,
+                      long s0, long s1, int form, cudaStream_t st, bool* used, bool* gated);
 
 namespace {
 
@@ -134,7 +135,8 @@ __device__ bool cta_wait_and(const int* flag, int target, int* err) {
 
 __global__ void __launch_bounds__(kChaseThreads)
     chase_kernel(int n, double* __restrict__ sub, double* __restrict__ U, long ldU, int* prog,
-                 int* ticket, int* err, int s_begin, int s_end) {
+                 int* ticket, int* err, const int* gate, int s_begin, int s_end) {
+  if (gate != nullptr && !(*(volatile const int*)gate & kGateShut)) return;
   __shared__ __align__(16) ChaseSmem sm;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(kChaseThreads)
     int rb = min(kBW, (int)(n - r));
     int cb = 1;  // columns of the previous tile (B1): 1 at the first step
     int cur = 0;
-    if (s > 0 && !cta_wait_and(prog + s - 1, (int)(r + 2 * kBW), err)) break;
+    if (s > s_begin && !cta_wait_and(prog + s - 1, (int)(r + 2 * kBW), err)) break;
     // previous tile = column s (its offsets 1..rb hold B1 = A(r:r+rb, s))
     tile_load_async(sm.tile[1 - cur], sub, s, 1);
     cp_async_commit_wait_all();
@@ -280,9 +282,9 @@ __global__ void __launch_bounds__(kChaseThreads)
       r = r2;
       cur = 1 - cur;
       // the next step's Householder warp reads B1 = this step's B1', written
-      // by all four warps in (6): the wait below ends with a CTA barrier; sweep
-      // 0 waits on nobody and takes the barrier alone
-      if (s > 0) {
+      // by all four warps in (6): the wait below ends with a CTA barrier; the
+      // first sweep waits on nobody and takes the barrier alone
+      if (s > s_begin) {
         if (!cta_wait_and(prog + s - 1, (int)(r + 2 * kBW), err)) {
           alive = false;
           break;
@@ -334,9 +336,9 @@ long chase_iwork_ints(long n) { return n + 64 + chase_pipe_ints(n); }
 
 // Sweeps [s0, s1) of the chase as one launch (part `part`, 0 <= part < 32, of
 // a chase split into consecutive ranges; part 0 starts at s0 = 0 and clears
-// the flags, tickets and error word).  Each part has its own ticket counter
-// (iwork[n + part]); a part's first sweep waits on the previous sweep's
-// progress flag, which the previous part's launch left at its final value.
+// the flags, tickets, gate and error word).  Each part has its own ticket
+// counter (iwork[n + part]); the first sweep of a part waits on nobody, since
+// the stream has the part before it done, by whichever kernel.
 // Splitting costs one pipeline drain per part boundary: the next part's
 // first sweep starts when the previous sweep has reached the end of the band,
 // not 2b rows after its start.
@@ -354,17 +356,19 @@ int chase_part_async(long n, long b, double* dSub, long ldSub, double* dU, long 
   if (part == 0) EVD_CUDA_TRY(cudaMemsetAsync(iwork, 0, sizeof(int) * chase_iwork_ints(n), st));
   s1 = std::min(s1, n - 2);
   if (s1 > s0) {
-    bool used = false;
-    if (form == kChaseAuto)
-      EVD_TRY(launch_chase_pipe(n, dSub, dU, ldU, err, iwork + n + 64, s0, s1, st, &used));
-    if (used) return EVD_SUCCESS;
+    int* gate = iwork + n + 33;
+    bool used = false, gated = false;
+    if (form != kChaseTicketed)
+      EVD_TRY(launch_chase_pipe(n, dSub, dU, ldU, err, iwork + n + 64, gate, s0, s1, form, st,
+                                &used, &gated));
+    if (used && !gated) return EVD_SUCCESS;
     // enough CTAs for the pipeline's concurrency (a sweep starts every 3 steps
     // and lasts about n/b steps), bounded by the GPU's resident capacity
     const long sweeps = s1 - s0;
     const long want = n / (3 * kBW) + 16;
     const int ctas = (int)std::min(std::min(sweeps, want), 6L * device_sm_count());
     chase_kernel<<<ctas, kChaseThreads, 0, st>>>((int)n, dSub, dU, ldU, prog, iwork + n + part,
-                                                 err, (int)s0, (int)s1);
+                                                 err, used ? gate : nullptr, (int)s0, (int)s1);
     EVD_LAUNCHED();
   }
   return EVD_SUCCESS;

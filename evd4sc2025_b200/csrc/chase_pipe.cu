@@ -35,8 +35,13 @@
 // Measured figures: at launch_chase_pipe, where the form is chosen.
 //
 // Progress: every slot waits for both neighbours, so all CTAs of a launch must
-// be resident together.  One CTA, one cluster (co-scheduled by definition) or
-// a cooperative launch guarantee that; every wait is bounded all the same.
+// be resident together.  One CTA and one cluster (co-scheduled by definition)
+// are.  A cooperative launch fits the device, but other kernels may hold the SMs
+// of some of its CTAs for any time (a long kernel on another stream, or two such
+// launches of different priority, each with a part of the SMs).  So its CTAs
+// first count themselves in at a gate; if they are not complete after 2 s the
+// gate shuts, all of them leave, and the ticketed kernel behind them, whose
+// progress asks for no residency, does the sweeps.  Every wait is bounded.
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -54,6 +59,7 @@ constexpr int kPOff = 2 * kPB;       // band-storage rows per column
 constexpr int kSlotThreads = 64;     // a warp for N, a warp for S
 constexpr int kExtraWarps = 3;       // head, u relay, column relay
 constexpr unsigned long long kPipeTimeoutNs = 4000000000ull;  // 4 s
+constexpr unsigned long long kGateNs = 2000000000ull;         // 2 s
 typedef unsigned long long u64;
 
 struct __align__(16) Word2 {
@@ -204,7 +210,25 @@ struct PipeArgs {
   long ldU;
   int* err;
   Boundary* bnd;  // gridDim.x - 1 of them (cooperative launch), or nullptr (cluster)
+  int* gate;      // of a cooperative launch
 };
+
+// Thread 0 of every CTA of a cooperative launch: true once all have come.  The
+// word holds their number; it is shut by a compare-and-swap on an incomplete
+// number, so all CTAs get the same answer.
+__device__ bool pass_gate(int* gate) {
+  atomicAdd(gate, 1);
+  u64 t0 = 0, t;
+  for (unsigned it = 1;; ++it) {
+    const int v = ld_acquire(gate);
+    if (v & kGateShut) return false;
+    if (v == (int)gridDim.x) return true;
+    if ((it & 255u) != 0) continue;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    if (t0 == 0) t0 = t;
+    if (t - t0 > kGateNs) atomicCAS(gate, v, v | kGateShut);
+  }
+}
 
 // The reflector of x (rows at and below the first one): u (this lane's entry),
 // its first entry and the element that replaces x_0.  x0 and nrm2 are uniform.
@@ -515,6 +539,7 @@ __global__ void __launch_bounds__(SL* kSlotThreads + 32 * kExtraWarps, 1)
   for (int e = tid; e < 2 * (kPB + 1); e += blockDim.x) headbox[e] = Word2{0, 0};
   if (cluster && gridDim.x > 1) cg::this_cluster().sync();
   else __syncthreads();
+  if (!cluster && !__syncthreads_and(tid != 0 || pass_gate(a.gate))) return;
 
   const int nslots = (a.n - 2 - a.s0) / kPB + 1;
   const int k0 = (int)blockIdx.x * SL;
@@ -620,8 +645,9 @@ bool chase_pipelined(long n, int sms) {
 }
 
 // Sweeps [s0, s1) by the pipeline; false in *used when no form of it fits (the
-// caller then runs chase_kernel).  msg: chase_pipe_ints(n) ints, zeroed before
-// the first part of a chase.
+// caller then runs chase_kernel), true in *gated when chase_kernel has to follow
+// for the case that the gate shuts.  msg: chase_pipe_ints(n) ints, zeroed like
+// the gate before the first part of a chase.
 // The form, by the number of CTAs of 4 slots: one CTA, a cluster (messages
 // through distributed shared memory), or a cooperative launch (through L2 and
 // a relay warp), which costs 0.3 us more per message; with 7 slots per CTA
@@ -631,10 +657,11 @@ bool chase_pipelined(long n, int sms) {
 //   4096: 36.5 -> 8.5 (2.1), 16384: 182 -> 34.5 (2.1), 20000: 52 (2.6).
 // Inside a cluster the N warp is busy all the time (2750 of 2900 cycles, 600 of
 // them the reduce-scatter of z); above, the messages through L2 are the rest.
-int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* msg, long s0,
-                      long s1, cudaStream_t st, bool* used) {
+int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* msg, int* gate,
+                      long s0, long s1, int form, cudaStream_t st, bool* used, bool* gated) {
   *used = true;
-  PipeArgs a{(int)n, (int)s0, (int)s1, sub, U, ldU, err, nullptr};
+  *gated = false;
+  PipeArgs a{(int)n, (int)s0, (int)s1, sub, U, ldU, err, nullptr, gate};
   const int slots = (int)((n - 2 - s0) / kPB) + 1;
   const int need = (slots + kSlA - 1) / kSlA;
   if (need <= 8 || (need <= 16 && cluster16_fits())) {
@@ -643,6 +670,10 @@ int launch_chase_pipe(long n, double* sub, double* U, long ldU, int* err, int* m
     return launch<kSlA>(a, c, false, st, used);
   }
   a.bnd = reinterpret_cast<Boundary*>(((uintptr_t)msg + 15) & ~(uintptr_t)15);
+  *gated = true;
+  if (s0 > 0) EVD_CUDA_TRY(cudaMemsetAsync(gate, 0, sizeof(int), st));  // an earlier part's
+  if (form == kChaseShut)  // its highest byte
+    EVD_CUDA_TRY(cudaMemsetAsync(reinterpret_cast<char*>(gate) + 3, kGateShut >> 24, 1, st));
   const int most = std::min(device_sm_count(), kMaxPipeCtas);
   if (need <= most) return launch<kSlA>(a, need, true, st, used);
   const int needb = (slots + kSlB - 1) / kSlB;

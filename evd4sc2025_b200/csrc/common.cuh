@@ -55,9 +55,16 @@ enum DeviceError : int {
   kDevTimeoutStrips = 5,
 };
 
-// Which kernel runs a chase: the pipeline where it fits, or (the tests, at orders
-// where the pipeline would run) always the kernel with ticketed sweeps.
-enum ChaseForm : int { kChaseAuto = 0, kChaseTicketed = 1 };
+// Which kernel runs a chase: the pipeline where it fits, or (for the tests, at
+// orders where the pipeline would run) always the kernel with ticketed sweeps,
+// or the pipeline with the gate of a cooperative launch shut from the start.
+enum ChaseForm : int { kChaseAuto = 0, kChaseTicketed = 1, kChaseShut = 2 };
+
+// The gate of a cooperative chase launch: its CTAs count themselves in, and the
+// word turns to kGateShut if they do not all come in time.  Then none of them
+// has touched the band, and the ticketed kernel, which every such launch is
+// followed by and which else returns at once, runs the sweeps.
+constexpr int kGateShut = 1 << 30;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

@@ -11,6 +11,7 @@ builds that relation with vector clocks from the kernel's own conditions
 """
 import ctypes as C
 import pathlib
+import random
 import re
 
 import pytest
@@ -139,3 +140,37 @@ def test_every_bounded_wait_leaves_its_loop_as_a_whole_warp():
     assert len(calls) == 1
     loop = src[src.rindex("for (", 0, calls[0]):calls[0]]
     assert "!__all_sync(0xffffffffu, ready())" in loop
+
+
+def test_the_gate_gives_every_cta_the_same_answer():
+    """pass_gate: count in, then poll; out of patience, try to shut the gate on
+    the number just read.  CTAs come, poll and lose patience in any order, and
+    every interleaving ends with one answer, which is yes only if all came."""
+    shut, ctas = 1 << 30, 5
+    rng = random.Random(1)
+    answers = set()
+    for _ in range(4000):
+        gate, read, got = 0, {}, {}
+        late = rng.random() < 0.5  # some run lets patience end early
+        while len(got) < ctas:
+            c = rng.randrange(ctas)
+            if c in got:
+                continue
+            if c not in read:
+                gate, read[c] = gate + 1, None  # atomicAdd
+            elif read[c] is None:
+                v = gate  # the poll
+                if v & shut:
+                    got[c] = False
+                elif v == ctas:
+                    got[c] = True
+                elif late and rng.random() < 0.3:
+                    read[c] = v
+            else:  # atomicCAS with the number read
+                if gate == read[c]:
+                    gate |= shut
+                read[c] = None
+        assert len(set(got.values())) == 1
+        answers.add(got[0])
+        assert not got[0] or gate == ctas
+    assert answers == {True, False}

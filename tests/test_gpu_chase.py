@@ -147,3 +147,47 @@ def test_chase_reports_an_error_of_the_stages_before_it(cuda, evdlib):
     assert _chase(evdlib, cuda, band, 0, word)[0] == -3  # EVD_ERR_TIMEOUT
     word.zero_()
     assert _chase(evdlib, cuda, band, 0, word)[0] == 0
+
+
+@pytest.mark.parametrize("n", [2200, 4200])
+def test_chase_whose_gate_shuts_is_done_by_the_ticketed_kernel(cuda, evdlib, n):
+    g = torch.Generator(device=cuda).manual_seed(n)
+    band = torch.zeros(n, 64, dtype=torch.float64, device=cuda)
+    for o in range(33):
+        band[: n - o, o] = torch.randn(n - o, generator=g, dtype=torch.float64, device=cuda)
+    want = _chase(evdlib, cuda, band, 1)
+    got = _chase(evdlib, cuda, band, 2)
+    assert want[0] == 0 and got[0] == 0
+    assert all(torch.equal(a, b) for a, b in zip(want[1:], got[1:]))
+
+
+def test_cooperative_chases_on_streams_at_once(cuda, evdlib):
+    """Together they ask for more SMs than there are; results as alone."""
+    import threading
+    orders = (12000, 9000, 2500, 11000, 4100, 10000)
+    bands, want = [], []
+    for n in orders:
+        g = torch.Generator(device=cuda).manual_seed(n)
+        band = torch.zeros(n, 64, dtype=torch.float64, device=cuda)
+        for o in range(33):
+            band[: n - o, o] = torch.randn(n - o, generator=g, dtype=torch.float64, device=cuda)
+        bands.append(band)
+        want.append(evdlib.bulge_chase(band.clone().t(), 32)[:2])
+    torch.cuda.synchronize()
+    got = [None] * len(orders)
+
+    def work(i):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            sub = bands[i].clone()
+            got[i] = evdlib.bulge_chase(sub.t(), 32, stream=s)[:2]
+            s.synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(orders))]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    torch.cuda.synchronize()
+    for band, a, b in zip(bands, want, got):
+        if not torch.equal(a[0], b[0]):  # a gate that shut: the ticketed kernel's bits
+            a = _chase(evdlib, cuda, band, 1)[1:3]
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
