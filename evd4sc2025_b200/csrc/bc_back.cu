@@ -780,7 +780,7 @@ long q2_flag_ints(long n, long ncols) {
   return 4 + ((n - 2 + kStrip - 1) / kStrip) * ((ncols + 31) / 32);
 }
 
-constexpr size_t kQ8Smem = (size_t)2 * (kYBuf + kVBuf) * sizeof(double);  // 4 CTAs fit an SM
+constexpr size_t kQ8Smem = (size_t)2 * (kYBuf + kVBuf) * sizeof(double);  // of 4 CTAs per SM; registers allow 3
 
 template <bool FWD, int NW, bool RANGE>
 int launch_q2_8(long n, long ncols, const double* U, long ldU, const double* Tg, double* X,
@@ -820,18 +820,20 @@ int launch_q2(long n, long ncols, const double* U, long ldU, const double* Tg, d
 // 51.9, 16384 x 16384 461 -> 410 (21.4 TFLOP/s of algorithm, 0.72 of the DMMA
 // rate with the parallelogram padding).  Without counters, the 16-column kernel
 // from 64 columns per SM on (n = 16384: 436 ms), the 8-column one below.  A
-// launch over every sweep without an identity start takes the kernels compiled
-// without the range logic.
+// launch over every sweep without an identity start, as the reverse application
+// always is, takes the kernels compiled without the range logic.
 template <bool FWD>
 int launch_q2_pre(long n, long ncols, const double* U, long ldU, const double* Tg, double* X,
                   long ldX, Q2Range rg, int* flags, int* err, cudaStream_t st) {
-  const bool whole = !rg.ident && rg.h0 == 0 && rg.h1 >= n - 2;
   if (n <= kStrip + 2) flags = nullptr;  // a single strip
-  if (!flags && ncols >= 64L * device_sm_count())
-    return whole ? launch_q2<FWD, true, false>(n, ncols, U, ldU, Tg, X, ldX, rg, st)
-                 : launch_q2<FWD, true, true>(n, ncols, U, ldU, Tg, X, ldX, rg, st);
-  return whole ? launch_q2_8<FWD, 4, false>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, err, st)
-               : launch_q2_8<FWD, 4, true>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, err, st);
+  const bool wide = !flags && ncols >= 64L * device_sm_count();
+  if constexpr (FWD) {
+    if (rg.ident || rg.h0 > 0 || rg.h1 < n - 2)
+      return wide ? launch_q2<true, true, true>(n, ncols, U, ldU, Tg, X, ldX, rg, st)
+                  : launch_q2_8<true, 4, true>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, err, st);
+  }
+  return wide ? launch_q2<FWD, true, false>(n, ncols, U, ldU, Tg, X, ldX, rg, st)
+              : launch_q2_8<FWD, 4, false>(n, ncols, U, ldU, Tg, X, ldX, rg, flags, err, st);
 }
 
 // -V fragments of the blocks of sweeps [h0, h1) in every strip.
@@ -864,6 +866,7 @@ int q2_apply_range(bool forward, long n, long ncols, const double* U, long ldU, 
   if (n > (1L << 30) || ncols > (1L << 30)) return EVD_ERR_INVALID_ARG;
   if (h0 < 0 || h0 % 8 != 0 || h1 < h0 || (h1 % 8 != 0 && h1 < n - 2)) return EVD_ERR_INVALID_ARG;
   if (ident && (!forward || ident_k > h0)) return EVD_ERR_INVALID_ARG;
+  if (!forward && (h0 != 0 || h1 < n - 2)) return EVD_ERR_INVALID_ARG;
   if (n < 3 || ncols == 0 || h0 >= n - 2 || h1 == h0) return EVD_SUCCESS;
   if (!U || !X) return EVD_ERR_INVALID_ARG;
   if (tbuf && ((uintptr_t)tbuf & 15)) return EVD_ERR_INVALID_ARG;
