@@ -534,6 +534,11 @@ __device__ __forceinline__ double reciprocal(double x) {
   return fma(r, fma(-x, r, 1.0), r);
 }
 
+__global__ void reciprocal_kernel(long n, const double* x, double* y) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i < n) y[i] = reciprocal(x[i]);
+}
+
 __device__ __forceinline__ void group_bar(int grp) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kHalf) : "memory");
 }
@@ -827,4 +832,12 @@ extern "C" int evd_test_tsqr_timeout(long m, double* A, long lda, double* R, dou
   EVD_TRY(launch_pdl(tsqr_up_kernel, nodes, kThreads, sizeof(UpSmem), stream, plan, A, lda, work,
                      R, (long)kNB));
   return read_device_error(panel_error_word(work), stream);
+}
+
+// For the tests: y = reciprocal(x) of the panel's LU, elementwise.
+extern "C" int evd_test_reciprocal(long n, const double* x, double* y, cudaStream_t stream) {
+  if (n <= 0) return EVD_SUCCESS;
+  evd::reciprocal_kernel<<<evd::ceil_div_i(n, 256), 256, 0, stream>>>(n, x, y);
+  EVD_LAUNCHED();
+  return EVD_SUCCESS;
 }

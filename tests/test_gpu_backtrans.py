@@ -186,3 +186,34 @@ def test_a_strip_wait_that_runs_out_marks_every_column(cuda, evdlib, n, ncols, d
     assert torch.isnan(Y).any(dim=0).all()
     # and the device goes on as before
     assert torch.equal(evdlib.bc_back_apply(X, U), ref)
+
+
+@pytest.mark.parametrize("n,ncols", [(100, 30), (700, 200)])
+def test_q2_apply_in_a_stream_capture(cuda, evdlib, n, ncols):
+    """A captured call takes no counters from the pool (it runs unpipelined) and
+    replays to what the call gives outside; calls beside the replays, with
+    counters, are not disturbed."""
+    g = torch.Generator(device=cuda).manual_seed(n)
+    sub = torch.zeros(n, 64, dtype=torch.float64, device=cuda)
+    for o in range(33):
+        sub[: n - o, o] = torch.randn(n - o, generator=g, dtype=torch.float64, device=cuda)
+    _, _, U = evdlib.bulge_chase(sub.t(), 32)
+    X0 = evdlib.to_cm(torch.randn(n, ncols, generator=g, dtype=torch.float64, device=cuda),
+                      device=cuda)
+    X, Y = evdlib.empty_cm(n, ncols, device=cuda), evdlib.empty_cm(n, ncols, device=cuda)
+    work = torch.empty(evdlib.lib().evd_bc_back_work_size(n), dtype=torch.float64, device=cuda)
+    Y.copy_(X0)
+    want = evdlib.bc_back_apply(Y, U).clone(memory_format=torch.preserve_format)
+    torch.cuda.synchronize()
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=s):
+        X.copy_(X0)
+        evdlib.bc_back_apply(X, U, work=work, stream=s)
+    for _ in range(3):
+        X.fill_(7.0)
+        Y.copy_(X0)
+        graph.replay()
+        evdlib.bc_back_apply(Y, U)
+        torch.cuda.synchronize()
+        assert (X - want).abs().max() <= 1e-13 * np.sqrt(n) * X0.abs().max()
+        assert torch.equal(Y, want)

@@ -75,3 +75,56 @@ def test_a_tree_wait_that_runs_out_is_reported_and_stays_visible(cuda, evdlib, m
     assert rc == 0
     Rr = O.tsqr(A.numpy())[1]
     assert np.abs(R.cpu().numpy() - Rr).max() <= 1e-12 * np.abs(Rr).max()
+
+
+def test_reciprocal_of_the_panel_lu(cuda, evdlib):
+    """Two Newton steps from the hardware's approximation (2^-20 or better): the
+    error left is the last rounding, so within one ulp of the division."""
+    import ctypes as C
+    rng = np.random.default_rng(1)
+    x = np.concatenate([rng.uniform(1.0, 2.0, 100000),  # the LU's pivots
+                        rng.choice([-1.0, 1.0], 100000) * 10.0 ** rng.uniform(-290, 290, 100000),
+                        2.0 ** np.arange(-960, 961), np.nextafter(2.0 ** np.arange(-960, 961), 0)])
+    xd = torch.from_numpy(x).to(cuda)
+    y = torch.empty_like(xd)
+    torch.cuda.synchronize()
+    assert evdlib.lib().evd_test_reciprocal(C.c_long(x.size), C.c_void_p(xd.data_ptr()),
+                                            C.c_void_p(y.data_ptr()), None) == 0
+    want = 1.0 / x
+    assert (np.abs(y.cpu().numpy() - want) <= np.spacing(np.abs(want))).all()
+
+
+def test_panel_and_band_reduction_in_a_stream_capture(cuda, evdlib):
+    """Captured, the chains of kernels with programmatic launches and the tree's
+    counters replay to the same bits."""
+    n, nb = 512, 128
+    A = evdlib.to_cm(torch.from_numpy(O.sym_gaussian(n, 5)), device=cuda)
+    names = ("OA", "dA", "W", "Y")
+    buf = {k: evdlib.zeros_cm(n, n, device=cuda) for k in names}
+    Z, R = evdlib.zeros_cm(n, nb, device=cuda), evdlib.zeros_cm(n, nb, device=cuda)
+    lw = evdlib.lib().evd_sy2sb_work_size(n, 32, nb)
+    work = torch.zeros(lw, dtype=torch.float64, device=cuda)
+
+    def reduce(stream):
+        buf["OA"].copy_(A)
+        buf["dA"].copy_(A)
+        buf["W"].zero_()
+        buf["Y"].zero_()
+        args = []
+        for t in (*(buf[k] for k in names), Z, R):
+            args.extend(evdlib._cm(t, "x"))
+        evdlib.call("evd_sy2sb", n, n, 32, nb, *args, evdlib._ptr(work), lw,
+                    evdlib._stream(stream))
+
+    reduce(None)
+    torch.cuda.synchronize()
+    want = [buf[k].clone() for k in ("dA", "W", "Y")]
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=s):
+        reduce(s)
+    for _ in range(3):
+        for k in names:
+            buf[k].fill_(7.0)
+        g.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(buf[k], w) for k, w in zip(("dA", "W", "Y"), want))

@@ -173,50 +173,43 @@ def test_mixed_chain_plan_applies_every_sweep_once(evdlib):
 
 
 # ---------------------------------------------------------------------------
-# Panel QR tile factorisation (evd4sc2025_b200/csrc/panel_qr.cu, tile_factor):
-# warp w owns columns w, w + 8, ...; the owner of column j + 1 publishes
-# reflector j + 1 with bar.arrive on barrier 1 + ((j + 1) & 3), every other
-# warp waits on barrier 1 + (j & 3) before applying reflector j.  A barrier
-# instance completes once all 8 warps have arrived (arrive or sync).
+# Panel QR tree (evd4sc2025_b200/csrc/panel_qr.cu, tsqr_up_kernel): a CTA takes a
+# node from the ticket, leaves first, and works on its columns in four groups; a
+# group of an inner node waits until all children have published theirs.  Each
+# node counts its publications up in its parent's counter of the group, and the
+# parent resets a counter after its wait.
 
-def _qr_barrier_program(w, nw=8, nb=32):
-    ops = [("arrive", 0)] if w == 0 else []
-    for j in range(nb):
-        if w != (j & 7):
-            ops.append(("sync", j))
-        if j + 1 < nb and w == ((j + 1) & 7):
-            ops.append(("arrive", j + 1))
-    return ops
+def _tree(m):
+    tiles = [(m + 127) // 128]
+    while tiles[-1] > 1:
+        tiles.append((32 * tiles[-1] + 127) // 128)
+    nodes = [(lev, i) for lev, t in enumerate(tiles) for i in range(t)]
+    return tiles, nodes
 
 
-def test_panel_qr_barrier_protocol_cannot_deadlock():
+def test_panel_tree_cannot_deadlock_and_leaves_its_counters_at_zero():
     import random
-    nw = 8
-    progs = [_qr_barrier_program(w) for w in range(nw)]
-    # every column's barrier gets exactly one arrival per warp
-    for j in range(32):
-        assert sorted(w for w in range(nw) for op in progs[w] if op[1] == j) == list(range(nw))
     rng = random.Random(3)
-    for _ in range(3000):
-        pc, arrived, current, waiting = [0] * nw, {}, {}, [None] * nw
-        while True:
-            for w in range(nw):
-                if waiting[w] is not None and len(arrived.get(waiting[w], ())) == nw:
-                    waiting[w] = None
-                    pc[w] += 1
-            run = [w for w in range(nw) if pc[w] < len(progs[w]) and waiting[w] is None]
-            if not run:
-                assert all(pc[w] == len(progs[w]) for w in range(nw)), "deadlock"
-                break
-            w = rng.choice(run)
-            op, j = progs[w][pc[w]]
-            bid = 1 + (j & 3)
-            open_j = current.get(bid)
-            # a barrier id is reused only after its previous instance completed
-            assert open_j is None or open_j == j or len(arrived[open_j]) == nw
-            current[bid] = j
-            arrived.setdefault(j, set()).add(w)
-            if op == "arrive":
-                pc[w] += 1
-            else:
-                waiting[w] = j
+    for m in (32, 128, 160, 544, 4128, 16384):
+        tiles, nodes = _tree(m)
+        for resident in (1, 2, 3, 40):  # CTAs that fit the GPU at a time
+            count = {}
+            ticket, running, done = 0, [], set()
+            while len(done) < len(nodes):
+                while len(running) < resident and ticket < len(nodes):
+                    running.append([nodes[ticket], 0])
+                    ticket += 1
+                ready = [r for r in running if r[0][0] == 0 or count.get((*r[0], r[1]), 0)
+                         == min(4, tiles[r[0][0] - 1] - 4 * r[0][1])]
+                assert ready, "deadlock"
+                r = rng.choice(ready)
+                (lev, i), grp = r
+                count[lev, i, grp] = 0
+                if lev + 1 < len(tiles):
+                    key = (lev + 1, i // 4, grp)
+                    count[key] = count.get(key, 0) + 1
+                r[1] += 1
+                if r[1] == 4:
+                    running.remove(r)
+                    done.add(r[0])
+            assert not any(count.values())
