@@ -61,21 +61,22 @@ __global__ void final_sum_kernel(int nparts, const double* __restrict__ partial,
 
 // Reduction partials of the metrics (8 KB, module scope): the reference gives
 // checkOrthogonality exactly an M x M work buffer, so the partial sums cannot
-// live there.  Calls that overlap on the GPU share it.
+// live there.  A call holds the device's lock from its first use of them until
+// it has read its sums, so calls of several host threads take turns.
 __device__ double g_metric_partials[kRedBlocks + 16];
 
 }  // namespace
 
 // Device address of g_metric_partials on the current device (the runtime keeps
-// one copy of the module per device), cached per device under a lock.
-static int metric_scratch(double** p) {
+// one copy of the module per device), cached per device, and that device's lock.
+static int metric_scratch(double** p, std::unique_lock<std::mutex>* turn) {
   constexpr int kMaxDev = 64;
-  static std::mutex mu;
+  static std::mutex mu[kMaxDev];
   static double* addr[kMaxDev] = {};
   int d = -1;
   EVD_CUDA_TRY(cudaGetDevice(&d));
   if (d < 0 || d >= kMaxDev) return EVD_ERR_INVALID_ARG;
-  std::lock_guard<std::mutex> lock(mu);
+  *turn = std::unique_lock<std::mutex>(mu[d]);
   if (addr[d] == nullptr) EVD_CUDA_TRY(cudaGetSymbolAddress((void**)&addr[d], g_metric_partials));
   *p = addr[d];
   return EVD_SUCCESS;
@@ -103,7 +104,8 @@ extern "C" int evd_check_orthogonality(long M, long N, const double* dA, long ld
   // (cublasDgemm(T, N, M, M, N, ...)); work holds the M x M product.
   EVD_TRY(evd::dgemm('t', 'n', M, M, N, 1.0, dA, ldA, dB, ldB, 0.0, work, M, stream));
   double* scratch = nullptr;
-  EVD_TRY(evd::metric_scratch(&scratch));
+  std::unique_lock<std::mutex> turn;
+  EVD_TRY(evd::metric_scratch(&scratch, &turn));
   EVD_TRY(evd::frob_norm_dev(M, M, work, M, 1.0, nullptr, 0, nullptr, scratch + 8, scratch,
                              stream));
   double h = 0.0;
@@ -119,7 +121,8 @@ extern "C" int evd_check_eig(long n, const double* A, long lda, const double* w,
     return EVD_ERR_INVALID_ARG;
   double* AX = work;  // n x n
   double* scratch = nullptr;
-  EVD_TRY(evd::metric_scratch(&scratch));
+  std::unique_lock<std::mutex> turn;
+  EVD_TRY(evd::metric_scratch(&scratch, &turn));
   double* sums = scratch;    // [0] resid^2 [1] ||A||^2 [2] orth^2
   double* part = scratch + 8;
   EVD_TRY(evd::dgemm('n', 'n', n, n, n, 1.0, A, lda, X, ldX, 0.0, AX, n, stream));

@@ -149,3 +149,28 @@ def test_non_finite_input_is_an_error(cuda, evdlib, bad):
     assert e.value.status < 0
     w, X, res, orth = _run(cuda, evdlib, O.sym_gaussian(n, seed=13), 64)
     assert res <= TOL_RES and orth <= TOL_ORT
+
+
+def test_checks_of_several_threads_take_turns(cuda, evdlib):
+    """evd_check_eig on streams at once gives each caller its own norms."""
+    import threading
+    problems = []
+    for n in (64, 300, 700, 1100):
+        A = evdlib.to_cm(torch.from_numpy(O.sym_gaussian(n, n)), device=cuda)
+        w, X = evdlib.syevd(A, 32, 64)
+        w[n // 2] += 1e-3 * n  # a residual of its own for each
+        problems.append((A, w, X, evdlib.check_eig(A, w, X)))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(A, w, X, want):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            for _ in range(40):
+                if evdlib.check_eig(A, w, X, stream=s) != want:
+                    wrong.append(A.shape[0])
+
+    threads = [threading.Thread(target=work, args=p) for p in problems]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not wrong
