@@ -159,7 +159,8 @@ __global__ void init_kernel(long n, long np, int s, const double* d, const doubl
 
 __device__ __forceinline__ double sign_of(double a, double b) { return (b >= 0.0) ? fabs(a) : -fabs(a); }
 
-// One warp per leaf: lane i holds d_i and e_i, every lane runs the scalar
+// Implicit QL iteration (the steps of EISPACK's tql2), one warp per leaf: lane i
+// holds d_i and e_i, every lane runs the scalar
 // recurrence on values broadcast by shuffles and applies the rotations to its
 // own row of the eigenvector matrix, which stands in shared memory (column c
 // of lane's row at z[c * 32 + lane]: no bank conflicts, no other lane's data).

@@ -335,8 +335,9 @@ ChainPlan chain_plan(long n, bool buffer, bool pipelined) {
 // For the heaviest column their lengths are k (n - k) + k^2 / 2 and
 // (n - k)^2 / 2 in units of sweep-strips, equal at k = (1 - sqrt(1/2)) n.
 // The chains used to follow the chase one sweep range behind; since the chase
-// takes 41 ms of the solve at n = 16384 (181 ms before the pipeline kernel)
-// running it first, alone and in one launch, is faster (876 against 948 ms).
+// takes 41 ms of the solve at n = 16384 (181 ms before the pipeline kernel) it
+// runs first, alone and in one launch (876 against 948 ms for the solve when the
+// two were compared; 805 now).
 //   main:   sy2sb (emulated trailing SYR2K) -> band pack -> chase -> D&C (own
 //           integer workspace; Z into W once the Q1 formation no longer reads W)
 //   side B: slab merge, Q1 formed explicitly (emulated)
@@ -442,9 +443,9 @@ static int syevd_mixed_core(long n, long b, long nb, const double* A, long lda, 
     NvtxRange r("evd_b200 stage-2 reflectors (side streams)");
     // The pipelined kernel's counters into Z and R (free after stage 1).  Where
     // the 64-column CTAs of the plain kernel fill the SMs it is the better
-    // neighbour of the divide and conquer and the Q1 formation: n = 16384 833 ms
-    // against 859 (three pipelined CTAs per SM leave them no room), 8192 176
-    // against 165.
+    // neighbour of the divide and conquer and the Q1 formation: the solve of
+    // n = 16384 takes 805 ms with it against 830 (three pipelined CTAs per SM
+    // leave them no room), 8192 158 against 155, 4096 44.2 against 42.8.
     const bool fits = n < 64L * device_sm_count() && q2_flags(n, n) > 0 &&
                       q2_flags(n, n) <= 2 * n * nb;
     int* fl[2] = {fits ? (int*)Z : nullptr, fits ? (int*)R : nullptr};
